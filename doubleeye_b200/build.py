@@ -17,7 +17,7 @@ CSRC = os.path.join(PKG, "csrc")
 OUT_DIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(OUT_DIR, "libdoubleeye_b200.so")
 
-SOURCES = ["de_dense.cu", "de_capi.cu", "de_noalloc.cu", "de_sparse.cu", "de_edges.cu",
+SOURCES = ["de_dense.cu", "de_cols.cu", "de_capi.cu", "de_noalloc.cu", "de_sparse.cu", "de_edges.cu",
            "de_serve.cu", "de_graph.cu", "de_prior.cu", "de_fill.cu"]
 # the bench's integer-pipe probe: its own library, outside the matcher's C ABI
 PROBE_SRC = "de_probe.cu"

@@ -101,6 +101,7 @@ void make_dev_cfg(const de_cfg& c, DevCfg* o) {
   o->min_ratio = c.min_ratio;
   o->expire_polls = de::get_expire_polls();
   o->cols_async = de::get_cols_async();
+  o->alone = 1;
   const int nbits = census_bits(c);
   o->packed = nbits <= 48;
   const int half = nbits / 2;
@@ -344,7 +345,8 @@ void part_batch(const de::Batch& b, int parts, int k, de::Batch* out) {
 
 int g_batch_streams = 2;          // parts a batch of several pairs is run as, 1..4
 
-int run_batch(const de_cfg& c, de::Batch& b, cudaStream_t s, int max_parts, bool reg_ring) {
+int run_batch(const de_cfg& c, de::Batch& b, cudaStream_t s, int max_parts, bool reg_ring,
+              bool overlapped) {
   de::DevCfg dc;
   de::make_dev_cfg(c, &dc);
   if (reg_ring) dc.cols_async = 0;
@@ -361,6 +363,7 @@ int run_batch(const de_cfg& c, de::Batch& b, cudaStream_t s, int max_parts, bool
   // Pairs are independent, so the results are the single chain's.  With stage timing
   // on, the stages run in order on the caller's stream.
   const int parts = std::min(b.n, max_parts);
+  dc.alone = parts <= 1 && !overlapped;
   PartStreams* ps = (!timed && parts > 1) ? part_streams(s) : nullptr;
   if (ps) {
     thread_local de::Batch sub;
@@ -476,7 +479,8 @@ int de_dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspace
 }  // extern "C"
 
 int de::dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspace,
-                  size_t ws_bytes, cudaStream_t stream, int max_parts, bool reg_ring) {
+                  size_t ws_bytes, cudaStream_t stream, int max_parts, bool reg_ring,
+                  bool overlapped) {
   size_t need = 0;
   int rc = de_dense_workspace_bytes(cfg, pairs, n, &need);
   if (rc) return rc;
@@ -496,7 +500,7 @@ int de::dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspac
     for (int i = 0; i < m; ++i)
       ws += de::pair_workspace_bytes(pairs[first + i].W, pairs[first + i].H,
                                      pair_D(*cfg, pairs[first + i]), cfg->lrc != 0);
-    if ((rc = run_batch(*cfg, b, s, max_parts, reg_ring))) return rc;
+    if ((rc = run_batch(*cfg, b, s, max_parts, reg_ring, overlapped))) return rc;
   }
   return DE_OK;
 }
@@ -977,7 +981,7 @@ int de_ctx_dense_batch(de_ctx* c, const de_pair* hp, int n) {
       // e2e 4990 -> 5045 pairs/s with the register ring here)
       if ((r = de::dense_dev(&c->cfg, dp.data() + bound[k], bound[k + 1] - bound[k],
                              dws + woff[k], woff[k + 1] - woff[k], sk,
-                             nch > 1 ? 1 : g_batch_streams, nch > 1)))
+                             nch > 1 ? 1 : g_batch_streams, nch > 1, nch > 1)))
         return r;
       DE_CUDA(cudaMemcpyAsync(&hstat[k], dws + woff[k], sizeof(int), cudaMemcpyDeviceToHost, sk));
       DE_CUDA(cudaEventRecord(c->ev_done[k], sk));

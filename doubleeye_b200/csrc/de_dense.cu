@@ -40,21 +40,13 @@
 #include <type_traits>
 #include <cuda_runtime.h>
 
+#include "de_dev.cuh"
 #include "de_internal.h"
 
 namespace de {
 namespace {
 
 constexpr float kNegBig = -1e30f;
-
-__device__ __forceinline__ int find_pair(const int* prefix, int n, int item) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (prefix[mid] <= item) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
 
 // One recursive-filter step (core/tools/de_dense.cpp:419): int32 carry, +2^14
 // rounding, arithmetic shift.
@@ -239,7 +231,9 @@ __global__ void __launch_bounds__(kCTX * kCTY) k_census_rows(DevCfg cfg, Batch b
 // at its first lane's start.  Values left of a plane's valid window never reach a
 // valid output (the vertical passes stay within a column and the top-2 masks
 // k > x - hw - dmin), so they are not computed exactly and not needed.
-// Score table: (h, m) -> Q14 score, h = Hamming distance, m = |L - R| clamped to
+// The volume holds scores with a bias of 32768 (the filter commutes with it), so that a
+// 16-bit value is one byte permute away from a float in the column kernel.
+// Score table: (h, m) -> Q14 score + bias, h = Hamming distance, m = |L - R| clamped to
 // TS-1 (exact: the AD score saturates at ad_trunc < TS).  Stored m-major with 64
 // h-entries per row, so the many lookups that share the saturated m read adjacent
 // entries, not one bank.
@@ -262,51 +256,7 @@ __device__ __forceinline__ int32_t graded(uint64_t lw, uint64_t rw, const void* 
     ad = abs(int(sLp[xl]) - int(sRp[xr]));
   }
   if (TS == 16) ad = min(ad, 15);
-  return static_cast<const int16_t*>(tab)[ad * 64 + h];
-}
-
-// Bulk asynchronous copies (cp.async.bulk, the TMA engine's 1-D form) with
-// mbarrier completion.  Every wait is bounded: if a phase never completes the
-// kernel records it in the batch status word and runs on to its end.
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-  return uint32_t(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes,
-                                          uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-constexpr int kWaitLimit = 1 << 22;                  // try_wait rounds before giving up
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int* err,
-                                          int limit = kWaitLimit) {
-  for (int i = 0; i < limit; ++i)
-    if (mbar_test(bar, parity)) return;
-  if (err) atomicExch(err, 1);
-}
-__device__ __forceinline__ void fence_proxy_async() {
-  asm volatile("fence.proxy.async;" ::: "memory");
+  return static_cast<const uint16_t*>(tab)[ad * 64 + h];
 }
 
 // One row per CTA iteration (the grid is persistent over rows); all pairs of a
@@ -322,6 +272,7 @@ __device__ __forceinline__ void fence_proxy_async() {
 // the per-stage barrier than an extra row gains (2 KB stages, nine rows per SM at
 // 848x480 D=128: rows 0.935 -> 0.971 ms per 16 pairs).
 constexpr int kRowsChunk = 2048;
+constexpr int kVolBias = 32768;
 
 template <bool PACKED, int TS, int G, int NS>
 __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
@@ -351,10 +302,11 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   {
-    int16_t* t16 = reinterpret_cast<int16_t*>(tabp);
+    uint16_t* t16 = reinterpret_cast<uint16_t*>(tabp);
     for (int i = tid; i < TS * 64; i += blockDim.x) {
       const int m = i >> 6, h = i & 63;
-      t16[i] = int16_t((int32_t(cfg.tbl[h]) * (1024 - cfg.wq) + int32_t(cfg.adt[m]) * cfg.wq) >> 10);
+      t16[i] = uint16_t(kVolBias +
+                        ((int32_t(cfg.tbl[h]) * (1024 - cfg.wq) + int32_t(cfg.adt[m]) * cfg.wq) >> 10));
     }
   }
   __syncthreads();
@@ -415,7 +367,7 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
     const int xw = hw + dmin + 2 * (tid & ~31);       // first lane's start in this warp
     const int xend = W - hw;                          // scores are 0 from here on
     uint32_t* out = reinterpret_cast<uint32_t*>(P.vol + row * DP) + tid;
-    int32_t f0 = 0, f1 = 0;
+    int32_t f0 = kVolBias, f1 = kVolBias;
     {
       uint64_t rprev = (xw - 1 - d0 >= 0) ? sR[xw - 1 - d0] : 0;    // chain k1's word
       int x = xw;
@@ -425,7 +377,7 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
       for (; x < xramp; ++x) {
         const int32_t a = sax[x];
         const uint64_t lw = sLx[x];
-        int32_t v0 = 0, v1 = 0;
+        int32_t v0 = kVolBias, v1 = kVolBias;
         uint64_t rw = 0;
         if (x - d0 >= hw) {
           rw = sR[x - d0];
@@ -473,8 +425,8 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
       }
       for (; x < W; ++x) {                            // right border, score 0
         const int32_t a = sax[x];
-        f0 = rf_step(0, f0, a);
-        f1 = rf_step(0, f1, a);
+        f0 = rf_step(kVolBias, f0, a);
+        f1 = rf_step(kVolBias, f1, a);
         out[x * XS] = pack2(f0, f1);
       }
     }
@@ -508,16 +460,16 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
         for (int q = CH - 1; q >= 0; --q) {
           const uint32_t c = cb[q * XS];
           const int32_t a = a1p[q];
-          g0 = rf_step(lo16(c), g0, a);
-          g1 = rf_step(hi16(c), g1, a);
+          g0 = rf_step(int32_t(c & 0xFFFFu), g0, a);
+          g1 = rf_step(int32_t(c >> 16), g1, a);
           o[q * XS] = pack2(g0, g1);
         }
       } else {
         for (int x = xhi; x >= xlo; --x) {
           const uint32_t c = cb[(x - xa) * XS];
           const int32_t a = sax[x + 1];
-          g0 = rf_step(lo16(c), g0, a);
-          g1 = rf_step(hi16(c), g1, a);
+          g0 = rf_step(int32_t(c & 0xFFFFu), g0, a);
+          g1 = rf_step(int32_t(c >> 16), g1, a);
           out[x * XS] = pack2(g0, g1);
         }
       }
@@ -535,10 +487,6 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
 }
 
 // ---------------------------------------------------------------------------------
-__device__ __forceinline__ int32_t sx16(uint32_t v) {     // sign-extended low half
-  return int32_t(int16_t(uint16_t(v & 0xFFFFu)));
-}
-__device__ __forceinline__ int32_t hx16(uint32_t v) { return int32_t(v) >> 16; }
 __device__ __forceinline__ uint32_t pk16(int32_t lo, int32_t hi) {
   return __byte_perm(uint32_t(lo), uint32_t(hi), 0x5410);
 }
@@ -622,7 +570,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
   // state and is still the fastest), 4 with a 4-deep ring, 2 at 16 disparities per
   // lane (more would spill)
   constexpr int kRB = KT >= 16 ? 2 : (PF >= 8 ? 8 : 4);
-  __shared__ __align__(16) int16_t sbuf[NT / 32][kRB][32 * KT];   // kRB row buffers per warp
+  __shared__ __align__(16) uint16_t sbuf[NT / 32][kRB][32 * KT];   // kRB row buffers per warp
   // AS: the prefetch ring in (dynamic) shared memory, PF slots of 16 bytes per lane,
   // so it costs no registers (more warps per SM) and no barrier (a lane reads only its
   // own slots); per warp, slot j of lane l is word (j * 32 + l) * KW
@@ -655,12 +603,13 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
   const uint16_t* ay = P.ay + (colok ? x : xbase);
   int32_t st[KT];
 #pragma unroll
-  for (int s = 0; s < KT; ++s) st[s] = 0;
+  for (int s = 0; s < KT; ++s) st[s] = kVolBias;      // v + 32768 throughout
+  constexpr uint32_t kZero2 = 0x80008000u;            // two zero scores of the volume
   auto step = [&](const uint32_t* w, int32_t a) {
 #pragma unroll
     for (int i = 0; i < KW; ++i) {
-      st[2 * i] = rf_step(sx16(w[i]), st[2 * i], a);
-      st[2 * i + 1] = rf_step(hx16(w[i]), st[2 * i + 1], a);
+      st[2 * i] = rf_step(int32_t(w[i] & 0xFFFFu), st[2 * i], a);
+      st[2 * i + 1] = rf_step(int32_t(w[i] >> 16), st[2 * i + 1], a);
     }
   };
   auto pack_state = [&](uint32_t* w) {
@@ -701,7 +650,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
     ring_take(j, c);
     const uint32_t dep = c[0];
 #pragma unroll
-    for (int i = 0; i < KW; ++i) c[i] = (y < yin) ? c[i] : 0u;
+    for (int i = 0; i < KW; ++i) c[i] = (y < yin) ? c[i] : kZero2;
     const int32_t a = aring[j];
     const int yn = y + PF;
     ring_fill(j, min(yn, ylast), dep);
@@ -736,7 +685,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
     step(c, ay[size_t(ys + 1) * W]);
   }
   if (ys < hh) return;
-  int16_t* rowbufs[kRB];
+  uint16_t* rowbufs[kRB];
 #pragma unroll
   for (int i = 0; i < kRB; ++i) rowbufs[i] = &sbuf[wib][i][gbase * KT];
   constexpr int kRowbufLast = TPCP * KT - 1;          // the group's last rowbuf entry
@@ -744,7 +693,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
     constexpr bool RK = decltype(with_rkey)::value;
     // One row: the filter step, the lane's top-2 keys, and its costs into a row
     // buffer (for the winner's neighbours).
-    auto row_keys = [&](int y, int j, uint32_t& pk0, uint32_t& pk1, int16_t* rowbuf) {
+    auto row_keys = [&](int y, int j, uint32_t& pk0, uint32_t& pk1, uint16_t* rowbuf) {
       uint32_t c[KW];
       ring_take(j, c);
       const int32_t a = aring[j];
@@ -754,20 +703,22 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
       step(c, a);
       pk0 = 0;
       pk1 = 0;                                        // key 0 never displaces a candidate
+      auto key_of = [&](int s) {
+        return (s < nvalid) ? (uint32_t(st[s]) << 8) | uint32_t(255 - k0 - s) : 0u;
+      };
 #pragma unroll
-      for (int s = 0; s < KT; ++s) {
-        const uint32_t key =
-            (s < nvalid) ? (uint32_t(st[s] + 32768) << 8) | uint32_t(255 - k0 - s) : 0u;
-        const uint32_t lo = min(pk0, key);
-        pk0 = max(pk0, key);
-        pk1 = max(pk1, lo);
+      for (int s = 0; s < KT; s += 2) {               // two keys at a time
+        const uint32_t ka = key_of(s), kb = key_of(s + 1);
+        const uint32_t sum = pk0 + ka + kb, hi = __vimax3_u32(pk0, ka, kb), lo = __vimin3_u32(pk0, ka, kb);
+        pk0 = hi;
+        pk1 = max(pk1, sum - hi - lo);
       }
       if (RK) {
         const size_t rowo = size_t(y) * W + x - dmin - k0;
 #pragma unroll
         for (int s = 0; s < KT; ++s)
           if (s < nvalid)
-            atomicMax(P.rkey + rowo - s, (uint32_t(st[s] + 32768) << 8) | uint32_t(255 - k0 - s));
+            atomicMax(P.rkey + rowo - s, (uint32_t(st[s]) << 8) | uint32_t(255 - k0 - s));
       }
       uint32_t o[KW];
       pack_state(o);
@@ -781,10 +732,10 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
       pk1 = max(max(pk1, o1), lo);
     };
     // a lane holding a row's merged keys writes them, with the winner's neighbours
-    auto emit = [&](int y, uint32_t pk0, uint32_t pk1, const int16_t* rowbuf) {
+    auto emit = [&](int y, uint32_t pk0, uint32_t pk1, const uint16_t* rowbuf) {
       const int kw = pk0 ? 255 - int(pk0 & 255u) : -1;
-      const int32_t vm = rowbuf[max(kw - 1, 0)];
-      const int32_t vp = rowbuf[min(kw + 1, kRowbufLast)];
+      const int32_t vm = int32_t(rowbuf[max(kw - 1, 0)]) - kVolBias;
+      const int32_t vp = int32_t(rowbuf[min(kw + 1, kRowbufLast)]) - kVolBias;
       const int32_t nm = (kw >= 1) ? vm : -32768;
       const int32_t np = (kw >= 0 && kw + 1 <= kmax) ? vp : -32768;
       const size_t i = size_t(y) * W + x;
@@ -1479,9 +1430,31 @@ cudaError_t launch_cols_g(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
   }
 }
 
+// Whether a disparity group goes to the tensor-memory column kernel.  Its time is per
+// tile (512 bytes of an image row, one tile an SM at a time, about 27 us at 480 rows) and
+// it fills an SM; the streaming kernel's grows with the bytes once the GPU is full.  They
+// cross between 6 and 11 tiles an SM (one launch set, streaming / this, us): 1280x720
+// D=128 (4.3 tiles an SM) 241 / 226, two 848x480 D=128 pairs (5.7) 175 / 153, 1280x720
+// D=256 (8.6) 381 / 376, four 848x480 D=128 pairs (11.4) 287 / 289.  A launch set that
+// runs beside others needs the room this kernel takes from them, and the reverse-match
+// keys (lrc) make its top-2 warps wait on atomics (848x480 D=64: 169 / 214): both stream.
+bool cols_tm_for(const DevCfg& cfg, const Batch& sub) {
+  if (!cfg.alone || sub.p[0].rkey) return false;
+  const int per = std::max(1, 256 / sub.maxDpad);     // columns per tile
+  int tiles = 0;
+  for (int i = 0; i < sub.n; ++i) {
+    if (!cols_tm_fits(sub.p[i].H, sub.maxDpad, cfg.hh)) return false;
+    tiles += (sub.cols_prefix[i + 1] - sub.cols_prefix[i] + per - 1) / per;
+  }
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return tiles <= 6 * nsm;
+}
+
 // One launch per disparity group present in the batch (Dpad = 64 G), so a pair's
 // column groups are sized for its own Dpad rather than the batch's largest, and each
-// group picks its tile shape from its own work.
+// group picks its kernel and tile shape from its own work.
 cudaError_t launch_cols(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
   if (b.cols_prefix[b.n] == 0) return cudaSuccess;
   thread_local Batch sub;
@@ -1497,7 +1470,8 @@ cudaError_t launch_cols(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
       ++sub.n;
     }
     if (sub.n == 0) continue;
-    const cudaError_t e = launch_cols_g(cfg, sub, s);
+    const cudaError_t e = cols_tm_for(cfg, sub) ? launch_cols_tm(cfg, sub, s)
+                                                : launch_cols_g(cfg, sub, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -28,7 +28,7 @@ struct DevPair {
   uint64_t* cwR;       //   element (y, x) at [y*cpitch + lpad + x] (left), [y*cpitch + x]
   uint16_t* ax;        // Q15 filter coefficients of L, x direction, [y*apitch + lpad + x]
   uint16_t* ay;        // ... y direction, [y*W + x]
-  int16_t* vol;        // [H][W][Dpad] filtered cost, int16 (Q14)
+  int16_t* vol;        // [H][W][Dpad] filtered cost, Q14 (+ 32768 outside the prior path)
   uint32_t* key0;      // packed top-2 keys, (v + 32768) << 8 | (255 - k); 0 = empty
   uint32_t* key1;
   uint32_t* nb;        // winner's neighbour costs, lo16 = k*-1, hi16 = k*+1 (-32768 none)
@@ -59,6 +59,7 @@ struct DevCfg {
   float lambda, gamma, damping, keep, min_margin, min_ratio;
   int expire_polls;    // test hook (knob "expire_wait_polls"), 0 = off
   int cols_async;      // column kernel's prefetch ring in shared memory (knob "cols_async")
+  int alone;           // the launch set runs by itself: small work may take whole SMs
   int16_t tbl[66];     // Q14 census score per Hamming distance
   int16_t adt[256];    // Q14 truncated-absolute-difference score
   uint16_t rf[256];    // Q15 filter coefficient per byte difference
@@ -77,9 +78,11 @@ struct Batch {
 
 // de_dense_dev with a bound on the parts a batch runs as on concurrent streams (1: one
 // launch set on `stream`); callers that already overlap batches of their own pass 1.
-// `reg_ring` keeps the column kernel's prefetch ring in registers (de_capi.cu).
+// `reg_ring` keeps the column kernel's prefetch ring in registers (de_capi.cu);
+// `overlapped`: the caller runs other launch sets beside this one.
 int dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspace,
-              size_t ws_bytes, cudaStream_t stream, int max_parts, bool reg_ring = false);
+              size_t ws_bytes, cudaStream_t stream, int max_parts, bool reg_ring = false,
+              bool overlapped = false);
 
 // Device address of the no-allocation entry point's status word on the current device
 // (de_noalloc.cu); DE_OK or an error code already recorded for de_last_error().
@@ -103,6 +106,10 @@ void parallel_copy(const std::vector<HostCopy>& jobs);
 cudaError_t launch_census(const DevCfg& cfg, const Batch& b, cudaStream_t s);
 cudaError_t launch_rows(const DevCfg& cfg, const Batch& b, cudaStream_t s);
 cudaError_t launch_cols(const DevCfg& cfg, const Batch& b, cudaStream_t s);
+// The column kernel with its forward results in tensor memory (de_cols.cu): one disparity
+// group's pairs, no reverse keys.  cols_tm_fits: its coefficient columns fit.
+bool cols_tm_fits(int H, int Dpad, int hh);
+cudaError_t launch_cols_tm(const DevCfg& cfg, const Batch& b, cudaStream_t s);
 cudaError_t launch_solve(const DevCfg& cfg, const Batch& b, bool from_ref_layout,
                          cudaStream_t s);
 void set_rows_ctas_per_sm(int v);

@@ -1,0 +1,31 @@
+"""The tensor-memory column kernel at the edges of its tiles, against the oracle bit for
+bit: 32-row blocks (a last block that is full, one row long, all border), the 512 rows
+that stay on chip and the ones that go back to the volume, tiles of 4, 2 and 1 columns
+that the image does not fill, and the four disparity groups with planes left over."""
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle, default_cfg
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("W,H,D", [
+    (8, 8, 1), (9, 9, 2), (41, 35, 31), (40, 36, 32), (97, 67, 64), (98, 70, 65),
+    (150, 38, 128), (151, 99, 100), (200, 40, 129), (210, 34, 192), (230, 33, 193),
+    (270, 45, 256), (31, 515, 12), (30, 516, 20), (45, 547, 33), (36, 610, 9), (90, 700, 70)])
+@pytest.mark.parametrize("hh", [3, 4])
+def test_tile_edges(W, H, D, hh):
+    from doubleeye_b200 import dense
+    rng = np.random.default_rng(W * 1000 + H)
+    L = rng.integers(0, 256, (H, W), dtype=np.uint8)
+    R = np.roll(L, -min(D, 5), 1) ^ rng.integers(0, 8, (H, W), dtype=np.uint8)
+    kw = dict(dmin=1, dmax=D, iters=2, census_hw=3, census_hh=hh)
+    got = dense.run_dense(L, R, dense.Cfg(**kw))
+    disp, margin, cand = Oracle().dense(default_cfg(**kw), L, R)
+    for name, a, b in (("disp", got.disp, disp), ("margin", got.margin, margin),
+                       *((f"plane {p}", got.cand[p], cand[p]) for p in range(6))):
+        same = (a.view(np.uint32) == b.view(np.uint32)) | (np.isnan(a) & np.isnan(b))
+        assert same.all(), f"{name}: {int((~same).sum())} values differ"
