@@ -24,7 +24,8 @@
 //             the winner's neighbour costs; rows stream through per-lane rings (in
 //             shared memory filled by cp.async at 8 disparities per lane, else in
 //             registers), with no block-wide step.
-//   k_solve   one CTA per row: candidate buckets by right pixel, damped max-sum
+//   k_solve_px, k_solve
+//             one CTA per row: the candidates of each right pixel, damped max-sum
 //             iterations, belief, and the one-to-one claim done in parallel as a
 //             per-right-pixel arg-max (each pixel claims exactly one right pixel,
 //             so "first in belief order wins" is that arg-max), sub-pixel fit,
@@ -36,6 +37,7 @@
 // be contracted, to match the reference's x86-64 single-precision results.
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 #include <cuda_runtime.h>
@@ -500,8 +502,8 @@ __device__ __forceinline__ uint32_t pk16(int32_t lo, int32_t hi) {
 // lane s of the group owns disparities [s*KT, s*KT + KT) as int16 pairs, so one row
 // of one column is 2*Dpad contiguous bytes, and adjacent columns are adjacent in
 // memory.  The top-2 key (v + 32768) << 8 | (255 - k) is unique per k, so the
-// strictly-greater insertion is three unsigned min/max, the merge across lanes is
-// four, and any merge order gives the sequential scan's answer.  The winner's
+// strictly-greater insertion of two keys is five unsigned operations, the merge across
+// lanes is four, and any merge order gives the sequential scan's answer.  The winner's
 // neighbour costs are read back from a per-group row buffer.
 //
 // No block-wide step: each lane reads its own 2*KT bytes of a row from global memory,
@@ -810,9 +812,10 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
 }
 
 // ---------------------------------------------------------------------------------
-// k_solve: the row solve, core/include/doubleeye/dense_solve.hpp:213-452 (K = 2,
-// candidates from the cost stage), plus the --out-conf planes and the confidence
-// (:158-171).  One CTA per row; shared-memory working set 49 bytes per pixel.
+// k_solve: the row solve, core/include/doubleeye/dense_solve.hpp:213-452 (K = 2), for
+// caller-made candidates and unbounded settings (else k_solve_px below), plus the
+// --out-conf planes and the confidence (:158-171).  One CTA per row; shared-memory
+// working set 49 bytes per pixel.
 
 
 __device__ __forceinline__ float fmax_ref(float a, float b) { return (a < b) ? b : a; }
@@ -825,6 +828,63 @@ __device__ float confidence_dev(float s1, float s2, float lambda, float lrc, flo
   const float logit = 0.692684f + 7.936751f * x;
   const float p = 1.f / (1.f + expf(-fmax_ref(-30.f, fmin_ref(30.f, logit))));
   return (lrc > tol) ? fmin_ref(p, 0.35f) : p;
+}
+
+// Sub-pixel offset of the winning candidate from its neighbours' costs (-32768: none);
+// dense_solve.hpp:389-434.
+__device__ __forceinline__ float fit_offset(const DevCfg& cfg, float c0, int32_t m16, int32_t p16) {
+  const float q = 1.f / 16384.f;
+  const float cm = (m16 == -32768) ? kNegBig : float(m16) * q;
+  const float cp = (p16 == -32768) ? kNegBig : float(p16) * q;
+  float off = 0.f;
+  if (cm > -1e29f && cp > -1e29f) {
+    const float den = cfg.fit_eq ? c0 - (cm < cp ? cm : cp) : 2.f * c0 - cm - cp;
+    if (den > 1e-6f) {
+      off = 0.5f * (cp - cm) / den;
+      off = off > 0.5f ? 0.5f : (off < -0.5f ? -0.5f : off);
+    }
+  }
+  return off;
+}
+
+// One pixel's outputs: disparity, reverse-match residuals (dense_solve.hpp:442-451,
+// core/tools/de_dense.cpp:1581-1597), candidate planes, confidence.  rev(xr): the
+// disparity index of the best candidate that names right pixel xr, -1 if none.
+template <typename Rev>
+__device__ __forceinline__ void put_pixel(const DevCfg& cfg, const DevPair& P, size_t row, int x,
+                                          int n, float s1, float s2, int k0, int k1, float dl,
+                                          Rev rev) {
+  const int W = P.W, dmin = cfg.dmin;
+  const size_t WH = size_t(W) * P.H;
+  if (P.disp) P.disp[row + x] = dl;
+  float lrc2 = __int_as_float(0x7fc00000);
+  float lrc = cfg.lrc ? __int_as_float(0x7fc00000) : kNegBig;
+  if (dl == dl) {
+    const int xr = x - int(lroundf(dl));
+    if (xr >= 0 && xr < W) {
+      const int k = rev(xr);
+      if (k >= 0) lrc2 = fabsf(dl - float(dmin + k));
+      if (cfg.lrc && P.rkey) {
+        const uint32_t rk = P.rkey[row + xr];
+        if (rk) lrc = fabsf(dl - float(dmin + 255 - int(rk & 255u)));
+      }
+    }
+  }
+  if (P.lrc2) P.lrc2[row + x] = lrc2;
+  if (P.cand) {
+    P.cand[row + x] = s1;
+    P.cand[WH + row + x] = s2;
+    P.cand[2 * WH + row + x] = n > 0 ? float(dmin + k0) : kNegBig;
+    P.cand[3 * WH + row + x] = n > 1 ? float(dmin + k1) : kNegBig;
+    P.cand[4 * WH + row + x] = lrc;
+    P.cand[5 * WH + row + x] = lrc2;
+  }
+  if (P.conf) {
+    uint8_t cv = 0;
+    if (dl == dl)
+      cv = uint8_t(lroundf(confidence_dev(s1, s2, cfg.lambda, (lrc2 == lrc2) ? lrc2 : 0.f, 1.f) * 255.f));
+    P.conf[row + x] = cv;
+  }
 }
 
 template <int kSolveThreads>
@@ -1093,9 +1153,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1536 / kSolveThreads) k_solve(D
     if (wx >= 0) s_win[wx] = 1;
   }
   __syncthreads();
-  // 7. outputs: disparity with sub-pixel fit (:380-434), reverse-match residuals
-  //    (:442-451, core/tools/de_dense.cpp:1581-1597), candidate planes, confidence
-  const size_t WH = size_t(W) * H;
+  // 7. outputs: disparity with sub-pixel fit (:380-434)
   auto outputs = [&](int x, uint32_t nb) {
     float dl = __int_as_float(0x7fc00000);
     const int n = s_cn[x];
@@ -1103,7 +1161,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1536 / kSolveThreads) k_solve(D
                                    n > 1 ? s_cs[s_pos[2 * x + 1]] : kNegBig);
     if (s_win[x]) {
       const int j = s_bestj[x];
-      const int d = dmin + s_cd[2 * x + j];
       float off = 0.f;
       if (cfg.subpixel && j == 0) {
         int32_t m16 = -32768, p16 = -32768;
@@ -1112,52 +1169,12 @@ __global__ void __launch_bounds__(kSolveThreads, 1536 / kSolveThreads) k_solve(D
         } else {
           m16 = lo16(nb); p16 = hi16(nb);
         }
-        const float c0 = cs2.x;
-        const float cm = (m16 == -32768) ? kNegBig : float(m16) * q;
-        const float cp = (p16 == -32768) ? kNegBig : float(p16) * q;
-        if (cm > -1e29f && cp > -1e29f) {
-          if (cfg.fit_eq) {
-            const float lower = cm < cp ? cm : cp;
-            const float den = c0 - lower;
-            if (den > 1e-6f) { off = 0.5f * (cp - cm) / den; off = off > 0.5f ? 0.5f : (off < -0.5f ? -0.5f : off); }
-          } else {
-            const float den = 2.f * c0 - cm - cp;
-            if (den > 1e-6f) { off = 0.5f * (cp - cm) / den; off = off > 0.5f ? 0.5f : (off < -0.5f ? -0.5f : off); }
-          }
-        }
+        off = fit_offset(cfg, cs2.x, m16, p16);
       }
-      dl = float(d) + off;
+      dl = float(dmin + s_cd[2 * x + j]) + off;
     }
-    if (P.disp) P.disp[row + x] = dl;
-    float lrc2 = __int_as_float(0x7fc00000);
-    float lrc = cfg.lrc ? __int_as_float(0x7fc00000) : kNegBig;
-    if (dl == dl) {
-      const int xr = x - int(lroundf(dl));
-      if (xr >= 0 && xr < W) {
-        if (s_rev[xr] >= 0) lrc2 = fabsf(dl - float(dmin + s_rev[xr]));
-        if (cfg.lrc && P.rkey) {
-          const uint32_t rk = P.rkey[row + xr];
-          if (rk) lrc = fabsf(dl - float(dmin + 255 - int(rk & 255u)));
-        }
-      }
-    }
-    if (P.lrc2) P.lrc2[row + x] = lrc2;
-    const float s1 = n > 0 ? cs2.x : kNegBig;
-    const float s2 = n > 1 ? cs2.y : kNegBig;
-    if (P.cand) {
-      P.cand[row + x] = s1;
-      P.cand[WH + row + x] = s2;
-      P.cand[2 * WH + row + x] = n > 0 ? float(dmin + s_cd[2 * x]) : kNegBig;
-      P.cand[3 * WH + row + x] = n > 1 ? float(dmin + s_cd[2 * x + 1]) : kNegBig;
-      P.cand[4 * WH + row + x] = lrc;
-      P.cand[5 * WH + row + x] = lrc2;
-    }
-    if (P.conf) {
-      uint8_t cv = 0;
-      if (dl == dl)
-        cv = uint8_t(lroundf(confidence_dev(s1, s2, lambda, (lrc2 == lrc2) ? lrc2 : 0.f, 1.f) * 255.f));
-      P.conf[row + x] = cv;
-    }
+    put_pixel(cfg, P, row, x, n, cs2.x, cs2.y, s_cd[2 * x], s_cd[2 * x + 1], dl,
+              [&](int xr) { return int(s_rev[xr]); });
   };
   // the neighbour words of a thread's pixels, four at a time, loads first
   const bool want_nb = !REF_LAYOUT && cfg.subpixel;
@@ -1171,6 +1188,276 @@ __global__ void __launch_bounds__(kSolveThreads, 1536 / kSolveThreads) k_solve(D
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (xb + u * kSolveThreads < W) outputs(xb + u * kSolveThreads, nb[u]);
+  }
+}
+
+// k_solve_px: the same solve with each pixel's state in its thread's registers, for the
+// cost stage's own candidates.
+//
+// k_solve keeps every candidate's score and messages in shared memory in bucket order and
+// looks its bucket up again each sweep; at 77% issue that was 35 M warp instructions a
+// 848x480 pair, about 230 lane instructions a pixel and sweep.  Here a thread owns NP pixels
+// of the row.  A pixel's rho needs only its own other candidate's beta: registers.  A
+// candidate's beta needs the rho of the other candidates of its right pixel: their places
+// are found once and kept, so a sweep writes two rho a pixel to shared memory and reads
+// the few it needs.  Right pixels named by at most four candidates (86% of the candidates
+// on slanted planes, 88-96% on most camera scenes) give each its three others, padded
+// with a place that holds -1e30; for the rest ("big") eight lanes a right pixel find the
+// greatest and the second (the greatest again on a tie) each sweep and update the
+// members' beta, which the owners fetch when they next need it.  Nothing is sorted or scanned: counts,
+// places and the one-to-one claim are shared-memory atomics whose result does not depend
+// on their order (the claim is the maximum belief, then the minimum x).
+//
+// What bounds it: issue (about 74%) and the two block barriers of a sweep.  Measured, the
+// solve stage at 16 848x480 D=128 pairs (us, k_solve -> this): 596 -> 385 at 8 sweeps,
+// 212 -> 114 at none; 48 -> 29 a sweep; one pair 64 -> 42, four 1500x1000 pairs at 12
+// sweeps 802 -> 591.  Of a sweep's 29 us the big right pixels are 9.
+//
+// Messages must stay finite for "the greatest of the others" to be free of order:
+// launch_solve keeps k_solve for any lambda, gamma or damping outside a bounded range,
+// and for caller-made candidates.
+constexpr int kSolveSmall = 4;           // members whose places the others keep
+
+__host__ __device__ constexpr int solve_big_max(int W) { return 2 * W / (kSolveSmall + 1) + 1; }
+
+__device__ __forceinline__ uint32_t ord_f32(float v) {    // order-preserving; -0 and +0 equal
+  const uint32_t b = __float_as_uint(v + 0.f);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
+template <int NP, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT > 512 ? 1 : NP == 2 ? 3 : 2) k_solve_px(DevCfg cfg, Batch b) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ int s_nbig, s_btot;
+  const int item = blockIdx.x;
+  const int pi = find_pair(b.solve_prefix, b.n, item);
+  const DevPair& P = b.p[pi];
+  const int W = P.W, H = P.H, NT = blockDim.x, tid = threadIdx.x;
+  const int y = item - b.solve_prefix[pi];
+  const int dmin = cfg.dmin, hw = cfg.hw;
+  const float lambda = cfg.lambda, gamma = cfg.gamma, damping = cfg.damping, keep = cfg.keep;
+  const int nbm = solve_big_max(W);
+  // shared bytes per pixel: places 8, rho 8, count 4, reverse key 4, big members 20, big
+  // right pixels 1.6.  A place is the byte offset of a candidate's rho.
+  uint2* s_mem = reinterpret_cast<uint2*>(smem);               // [W] four places of 16 bits
+  float* s_rho = reinterpret_cast<float*>(s_mem + W);          // [2W] by 2x + j, [2W] = -1e30
+  int* s_cnt = reinterpret_cast<int*>(s_rho + 2 * W + 2);      // [W] members, then kBig | index
+  uint32_t* s_rev = reinterpret_cast<uint32_t*>(s_cnt + W);    // [W] best score, first place
+  int* s_bo = reinterpret_cast<int*>(s_rev + W);               // [nbm] first member | members << 16
+  float* s_bcs = reinterpret_cast<float*>(s_bo + nbm);         // [2W] big members: score,
+  float* s_bbeta = s_bcs + 2 * W;                              // [2W] beta,
+  uint16_t* s_bmem = reinterpret_cast<uint16_t*>(s_bbeta + 2 * W);   // [2W] place
+  uint32_t* s_best = reinterpret_cast<uint32_t*>(s_rho);       // [W] after the sweeps
+  int* s_minx = reinterpret_cast<int*>(s_rho + W);             // [W] after the sweeps
+  constexpr int kBig = 1 << 16;
+  const bool row_ok = y >= cfg.hh && y < H - cfg.hh;
+  const size_t row = size_t(y) * W;
+  const float q = 1.f / 16384.f;
+  const uint32_t none = 8 * W;           // the place that holds -1e30
+
+  uint32_t key[NP][2];                   // (v + 32768) << 8 | 255 - k, 0 = no candidate
+  float cs[NP][2], beta[NP][2], rho[NP][2];
+  uint32_t oth[NP][2][2];                // places o1 | o2 << 16, o3; big: its member's offset
+  uint32_t big = 0;                      // which of the candidates' right pixels are big
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int x = tid + i * NT;
+    const bool ok = row_ok && x >= hw + dmin && x < W - hw;
+    key[i][0] = ok ? P.key0[row + x] : 0u;
+    key[i][1] = ok ? P.key1[row + x] : 0u;
+    if (x < W) {
+      s_cnt[x] = 0;
+      s_rev[x] = 0;
+    }
+  }
+  if (tid == 0) { s_nbig = 0; s_btot = 0; s_rho[2 * W] = kNegBig; }
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int x = tid + i * NT;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      cs[i][j] = key[i][j] ? float(int32_t(key[i][j] >> 8) - 32768) * q : kNegBig;
+      beta[i][j] = rho[i][j] = 0.f;
+    }
+    const float alt = key[i][1] ? fmax_ref(cs[i][1], lambda) : lambda;
+    if (P.margin && x < W) P.margin[row + x] = key[i][0] ? cs[i][0] - alt : 0.f;
+  }
+  auto right = [&](int i, int j) {       // the right pixel that a candidate names
+    return tid + i * NT - dmin - 255 + int(key[i][j] & 255u);
+  };
+  if (row_ok) {
+    __syncthreads();
+    // members of each right pixel, and the best score that names it (first place on ties)
+    uint32_t rank[NP][2];
+#pragma unroll
+    for (int i = 0; i < NP; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        rank[i][j] = 0;
+        if (!key[i][j]) continue;
+        const int xr = right(i, j), me = 2 * (tid + i * NT) + j;
+        if (cfg.iters > 0) rank[i][j] = uint32_t(atomicAdd(&s_cnt[xr], 1));
+        atomicMax(&s_rev[xr], (key[i][j] >> 8) << 13 | uint32_t(8191 - me));
+      }
+    __syncthreads();
+    if (cfg.iters > 0) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const int xr = tid + i * NT, c = xr < W ? s_cnt[xr] : 0;
+        if (c > kSolveSmall) {
+          const int g = atomicAdd(&s_nbig, 1), o = atomicAdd(&s_btot, c);
+          s_bo[g] = o | c << 16;
+          s_cnt[xr] = kBig | g;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (!key[i][j]) continue;
+          const int xr = right(i, j), c = s_cnt[xr], me = 2 * (tid + i * NT) + j;
+          if (c & kBig) {
+            const int p = (s_bo[c & 0xFFFF] & 0xFFFF) + int(rank[i][j]);
+            s_bmem[p] = uint16_t(4 * me);
+            s_bcs[p] = cs[i][j];
+            s_bbeta[p] = 0.f;
+            rank[i][j] = uint32_t(4 * p);
+            big |= 1u << (2 * i + j);
+          } else {
+            reinterpret_cast<uint16_t*>(s_mem + xr)[rank[i][j]] = uint16_t(4 * me);
+          }
+        }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t r = rank[i][j];
+          oth[i][j][1] = none;
+          if (!key[i][j] || big >> (2 * i + j) & 1) {   // (a big one's beta is its member's)
+            oth[i][j][0] = key[i][j] ? r | r << 16 : none | none << 16;
+            continue;
+          }
+          const int xr = right(i, j), c = s_cnt[xr];
+          const uint2 m = s_mem[xr];
+          const uint32_t m0 = m.x & 0xFFFFu, m1 = c > 1 ? m.x >> 16 : none;
+          const uint32_t m2 = c > 2 ? m.y & 0xFFFFu : none, m3 = c > 3 ? m.y >> 16 : none;
+          oth[i][j][0] = (r == 0 ? m1 : m0) | (r <= 1 ? m2 : m1) << 16;
+          oth[i][j][1] = r <= 2 ? m3 : m2;
+        }
+      const int nbig = s_nbig;
+      auto at = [](const float* a, uint32_t byte) {
+        return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(a) + byte);
+      };
+      auto big_betas = [&]() {
+#pragma unroll
+        for (int i = 0; i < NP; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            if (big >> (2 * i + j) & 1) beta[i][j] = at(s_bbeta, oth[i][j][0] & 0xFFFFu);
+      };
+      for (int it = 0; it < cfg.iters; ++it) {
+        if (it > 0) big_betas();
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          const float a0 = key[i][1] ? fmaxf(lambda, beta[i][1]) : lambda;
+          rho[i][0] = keep * (cs[i][0] - a0) + damping * rho[i][0];
+          rho[i][1] = keep * (cs[i][1] - fmaxf(lambda, beta[i][0])) + damping * rho[i][1];
+          if (key[i][0])
+            *reinterpret_cast<float2*>(s_rho + 2 * (tid + i * NT)) = make_float2(rho[i][0], rho[i][1]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NP; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float ex = fmaxf(fmaxf(at(s_rho, oth[i][j][0] & 0xFFFFu), at(s_rho, oth[i][j][0] >> 16)),
+                                   at(s_rho, oth[i][j][1]));
+            beta[i][j] = keep * (cs[i][j] - fmaxf(gamma, ex)) + damping * beta[i][j];
+          }
+        const int l = tid & 7;
+        const unsigned mask = 0xFFu << (tid & 24);
+        for (int g = tid >> 3; g < nbig; g += NT >> 3) {
+          const int o = s_bo[g] & 0xFFFF, end = o + (s_bo[g] >> 16), p0 = o + l;
+          const float v0 = at(s_rho, p0 < end ? uint32_t(s_bmem[p0]) : none);
+          float m1 = v0, m2 = kNegBig;
+          for (int p = p0 + 8; p < end; p += 8) {
+            const float v = at(s_rho, s_bmem[p]);
+            m2 = fmaxf(m2, fminf(m1, v));
+            m1 = fmaxf(m1, v);
+          }
+#pragma unroll
+          for (int h = 4; h > 0; h >>= 1) {
+            const float v1 = __shfl_xor_sync(mask, m1, h), v2 = __shfl_xor_sync(mask, m2, h);
+            m2 = fmaxf(fmaxf(m2, v2), fminf(m1, v1));
+            m1 = fmaxf(m1, v1);
+          }
+          auto update = [&](int p, float v) {
+            const float ex = v == m1 ? m2 : m1;
+            s_bbeta[p] = keep * (s_bcs[p] - fmaxf(gamma, ex)) + damping * s_bbeta[p];
+          };
+          if (p0 < end) update(p0, v0);
+          for (int p = p0 + 8; p < end; p += 8) update(p, at(s_rho, s_bmem[p]));
+        }
+        __syncthreads();
+      }
+      big_betas();
+    }
+  }
+  // belief (:343-358) and the gates (:364-374) folded into eligibility
+  float best[NP];
+  int bj[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    best[i] = kNegBig;
+    bj[i] = -1;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float c = cs[i][j];
+      if (!key[i][j] || c <= lambda) continue;
+      const float bel = (cfg.iters > 0) ? (beta[i][j] + rho[i][j] - c) : c;
+      if (bel > best[i]) { best[i] = bel; bj[i] = j; }
+    }
+    const float alt = key[i][1] ? fmax_ref(cs[i][1], lambda) : lambda;
+    if (cfg.min_margin > 0.f && cs[i][0] - alt < cfg.min_margin) bj[i] = -1;
+    if (cfg.min_ratio > 0.f && (1.f - alt) / fmax_ref(1.f - cs[i][0], 1e-6f) < cfg.min_ratio) bj[i] = -1;
+    const int x = tid + i * NT;
+    if (x < W) { s_best[x] = 0; s_minx[x] = W; }
+  }
+  // one-to-one claim (:359-378): per right pixel the claimant first in (belief desc, x asc)
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+    if (bj[i] >= 0) atomicMax(&s_best[right(i, bj[i])], ord_f32(best[i]));
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+    if (bj[i] >= 0 && s_best[right(i, bj[i])] == ord_f32(best[i]))
+      atomicMin(&s_minx[right(i, bj[i])], tid + i * NT);
+  __syncthreads();
+  uint32_t nb[NP];
+  bool win[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    win[i] = bj[i] >= 0 && s_minx[right(i, bj[i])] == tid + i * NT;
+    nb[i] = win[i] && cfg.subpixel && bj[i] == 0 ? P.nb[row + tid + i * NT] : 0x80008000u;
+  }
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int x = tid + i * NT;
+    if (x >= W) continue;
+    const int k0 = 255 - int(key[i][0] & 255u), k1 = 255 - int(key[i][1] & 255u);
+    float dl = __int_as_float(0x7fc00000);
+    if (win[i]) {
+      const float off = cfg.subpixel && bj[i] == 0 ? fit_offset(cfg, cs[i][0], lo16(nb[i]), hi16(nb[i])) : 0.f;
+      dl = float(dmin + (bj[i] ? k1 : k0)) + off;
+    }
+    put_pixel(cfg, P, row, x, int(key[i][0] != 0) + int(key[i][1] != 0), cs[i][0], cs[i][1], k0, k1,
+              dl, [&](int xr) {
+                const uint32_t r = s_rev[xr];
+                return r ? (8191 - int(r & 8191u)) / 2 - dmin - xr : -1;
+              });
   }
 }
 
@@ -1215,6 +1502,7 @@ size_t rows_smem(const Batch& b, int TS, int G, bool packed, int ring) {
 }
 
 size_t solve_smem(int W) { return size_t(W) * 49 + 64; }
+size_t solve_px_smem(int W) { return size_t(W) * 44 + 8 + size_t(solve_big_max(W)) * 4 + 16; }
 
 template <typename K>
 cudaError_t set_smem(K kernel, size_t bytes) {
@@ -1485,8 +1773,28 @@ cudaError_t launch_solve_w(const DevCfg& cfg, const Batch& b, bool from_ref, cud
   if (items == 0) return cudaSuccess;
   int maxW = 0;
   for (int i = 0; i < b.n; ++i) maxW = maxW > b.p[i].W ? maxW : b.p[i].W;
-  const size_t sm = solve_smem(maxW);
   cudaError_t e;
+  // the register kernel's messages stay bounded: finite terms, a damping of 0..1
+  const bool tame = fabsf(cfg.lambda) <= 1e6f && fabsf(cfg.gamma) <= 1e6f && cfg.damping >= 0.f &&
+                    cfg.damping <= 1.f;
+  if (!from_ref && tame) {
+    const size_t sm = solve_px_smem(maxW);
+    // pixels a thread: two up to 1024 pixels (40 registers, three CTAs an SM at 848; one
+    // 320x240 pair 21 us against 28 with four), four above, where two would leave one
+    // 1024-thread CTA an SM (1500x1000 D=256 x4: 624 us with two, 591 with four)
+    const int np = g_solve_threads ? (g_solve_threads == 512 ? 2 : 4) : (maxW <= 1024 ? 2 : 4);
+    auto go = [&](auto kern, int np) -> cudaError_t {
+      const cudaError_t e2 = set_smem(kern, sm);
+      if (e2 != cudaSuccess) return e2;
+      kern<<<items, ((maxW + np - 1) / np + 31) / 32 * 32, sm, s>>>(cfg, b);
+      return cudaGetLastError();
+    };
+    if (np == 2 && maxW <= 1024) return go(k_solve_px<2, 512>, 2);
+    if (np == 2 && maxW <= 2048) return go(k_solve_px<2, 1024>, 2);
+    if (maxW <= 2048) return go(k_solve_px<4, 512>, 4);
+    return go(k_solve_px<4, 1024>, 4);
+  }
+  const size_t sm = solve_smem(maxW);
   auto go = [&](auto kern, int nt) -> cudaError_t {
     cudaError_t e2 = set_smem(kern, sm);
     if (e2 != cudaSuccess) return e2;
