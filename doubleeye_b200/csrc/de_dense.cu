@@ -50,17 +50,8 @@ namespace {
 
 constexpr float kNegBig = -1e30f;
 
-// One recursive-filter step (core/tools/de_dense.cpp:419): int32 carry, +2^14
-// rounding, arithmetic shift.
-__device__ __forceinline__ int32_t rf_step(int32_t c, int32_t f, int32_t a) {
-  return c + ((a * (f - c) + (1 << 14)) >> 15);
-}
-
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
 
-__device__ __forceinline__ uint32_t pack2(int32_t lo, int32_t hi) {
-  return (uint32_t(uint16_t(lo))) | (uint32_t(hi) << 16);
-}
 __device__ __forceinline__ int32_t lo16(uint32_t v) { return int32_t(int16_t(v & 0xFFFFu)); }
 __device__ __forceinline__ int32_t hi16(uint32_t v) { return int32_t(int16_t(v >> 16)); }
 
@@ -68,15 +59,6 @@ __device__ __forceinline__ int32_t hi16(uint32_t v) { return int32_t(int16_t(v >
 // Census words + coefficient planes.
 // core/tools/de_dense.cpp:94-129,186-227 (census), :531-561 (rf_coeffs).
 constexpr int kCTX = 32, kCTY = 8, kMaxHalf = 4;
-
-// Packed census words (windows of <= 48 bits): lo32 = bits 0..31; hi32 = bits
-// 32..47 | guard bit 19 (left words only) | pixel byte at bits 20..27.  Then
-// (left.hi - right.hi) >> 20 is exactly L - R: the guard keeps the census bits from
-// borrowing into the pixel field.  (left ^ right) masked to the census bits gives the
-// Hamming input as before.
-constexpr uint32_t kCensusHiMask = 0xFFFFu;
-constexpr uint32_t kGuard = 1u << 19;
-constexpr int kPixShift = 20;
 
 __device__ __forceinline__ void census_generic(const uint8_t (*sL)[kCTX + 2 * kMaxHalf],
                                                const uint8_t (*sR)[kCTX + 2 * kMaxHalf],
@@ -233,34 +215,6 @@ __global__ void __launch_bounds__(kCTX * kCTY) k_census_rows(DevCfg cfg, Batch b
 // at its first lane's start.  Values left of a plane's valid window never reach a
 // valid output (the vertical passes stay within a column and the top-2 masks
 // k > x - hw - dmin), so they are not computed exactly and not needed.
-// The volume holds scores with a bias of 32768 (the filter commutes with it), so that a
-// 16-bit value is one byte permute away from a float in the column kernel.
-// Score table: (h, m) -> Q14 score + bias, h = Hamming distance, m = |L - R| clamped to
-// TS-1 (exact: the AD score saturates at ad_trunc < TS).  Stored m-major with 64
-// h-entries per row, so the many lookups that share the saturated m read adjacent
-// entries, not one bank.
-template <int TS, int CP>
-struct ScoreTable {
-  __host__ __device__ static constexpr size_t bytes() { return size_t(TS) * 64 * 2; }
-};
-
-template <bool PACKED, int TS, int CP>
-__device__ __forceinline__ int32_t graded(uint64_t lw, uint64_t rw, const void* tab,
-                                          const uint8_t* sLp, const uint8_t* sRp, int xl,
-                                          int xr) {
-  int h, ad;
-  if (PACKED) {
-    const uint32_t lh = uint32_t(lw >> 32), rh = uint32_t(rw >> 32);
-    h = __popc(uint32_t(lw) ^ uint32_t(rw)) + __popc((lh ^ rh) & kCensusHiMask);
-    ad = abs((int32_t(lh) - int32_t(rh)) >> kPixShift);
-  } else {
-    h = __popcll(lw ^ rw);
-    ad = abs(int(sLp[xl]) - int(sRp[xr]));
-  }
-  if (TS == 16) ad = min(ad, 15);
-  return static_cast<const uint16_t*>(tab)[ad * 64 + h];
-}
-
 // One row per CTA iteration (the grid is persistent over rows); all pairs of a
 // launch share Dpad = 64 G, so strides and chunk sizes are compile-time.  The row's
 // census words arrive by bulk copy into a single buffer that is refilled for the
@@ -274,7 +228,6 @@ __device__ __forceinline__ int32_t graded(uint64_t lw, uint64_t rw, const void* 
 // the per-stage barrier than an extra row gains (2 KB stages, nine rows per SM at
 // 848x480 D=128: rows 0.935 -> 0.971 ms per 16 pairs).
 constexpr int kRowsChunk = 2048;
-constexpr int kVolBias = 32768;
 
 template <bool PACKED, int TS, int G, int NS>
 __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
@@ -303,14 +256,7 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
     for (int i = 0; i < 4 + NS; ++i) mbar_init(&bars[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  {
-    uint16_t* t16 = reinterpret_cast<uint16_t*>(tabp);
-    for (int i = tid; i < TS * 64; i += blockDim.x) {
-      const int m = i >> 6, h = i & 63;
-      t16[i] = uint16_t(kVolBias +
-                        ((int32_t(cfg.tbl[h]) * (1024 - cfg.wq) + int32_t(cfg.adt[m]) * cfg.wq) >> 10));
-    }
-  }
+  fill_scores<TS>(cfg, tabp);
   __syncthreads();
   const void* tab = static_cast<const void*>(tabp);
   const int hw = cfg.hw, dmin = cfg.dmin;

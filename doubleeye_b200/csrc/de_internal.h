@@ -28,7 +28,7 @@ struct DevPair {
   uint64_t* cwR;       //   element (y, x) at [y*cpitch + lpad + x] (left), [y*cpitch + x]
   uint16_t* ax;        // Q15 filter coefficients of L, x direction, [y*apitch + lpad + x]
   uint16_t* ay;        // ... y direction, [y*W + x]
-  int16_t* vol;        // [H][W][Dpad] filtered cost, Q14 (+ 32768 outside the prior path)
+  int16_t* vol;        // [H][W][Dpad] filtered cost, Q14 + 32768
   uint32_t* key0;      // packed top-2 keys, (v + 32768) << 8 | (255 - k); 0 = empty
   uint32_t* key1;
   uint32_t* nb;        // winner's neighbour costs, lo16 = k*-1, hi16 = k*+1 (-32768 none)

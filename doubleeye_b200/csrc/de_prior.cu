@@ -11,24 +11,28 @@
 // full-plane filter there) and inserts the plane into a pixel's top-2 only inside the
 // row intervals.  Sub-pixel refinement is off under a prior (the tool turns it off).
 //
-// Layout here: the plane-minor volume [y][x][Dpad] of the dense path, so threads of a
-// warp take 32 consecutive planes of one row (or column) and every step of their
-// sequential chains touches 64 contiguous bytes.  Planes are independent until the
-// top-2, which is merged per pixel with a 64-bit compare-and-swap on two packed keys
-// ((v + 32768) << 8 | (255 - k), unique per plane), so the insertion order does not
-// matter.
-
+// Layout here: the plane-minor volume [y][x][Dpad] of the dense path.  Rows: a CTA per
+// image row with its census words in shared memory, a thread per pair of planes.
+// Columns: a group of lanes per column, four or eight planes a lane, whose top-2 are
+// merged over the group.  Each plane's rectangle enters as its own filter coefficient: 0
+// at the rectangle's first pixel takes the input as it is, 2^15 outside carries the state
+// through, both exactly, so all planes of a thread step together without branches.
+//
+// What bounds them: the serial chains at few warps an SM (one pair).  848x480 D=128, band
+// 2 (us, rows / columns): 888 / 1072 with a thread per plane, its loads in the chain, a
+// constant-memory score table and a compare-and-swap per insert; 200 / 247 now.
 #include <algorithm>
 
 #include <cuda_runtime.h>
 
+#include "de_dev.cuh"
 #include "de_internal.h"
 
 namespace de {
 namespace {
 
 constexpr int kMaskPad = 8;          // core/tools/de_dense.cpp:857 (MPAD)
-constexpr int kCasLimit = 1 << 20;   // retries of one top-2 merge before giving up
+constexpr int kHold = 1 << 15;       // the coefficient that leaves a state as it is
 
 struct Rect { int ylo, yhi, xlo, xhi, pylo, pyhi; };
 
@@ -45,12 +49,8 @@ __device__ __forceinline__ bool plane_rect(const int* box, int D, int k, int W, 
   return r->yhi - r->ylo >= 1 && r->xhi - r->xlo >= 2;
 }
 
-__global__ void k_prior_init(int* box, int D, int W, int H, unsigned long long* top2,
-                             long long WH) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < WH;
-       i += (long long)gridDim.x * blockDim.x)
-    top2[i] = 0ull;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < D; k += gridDim.x * blockDim.x) {
+__global__ void k_prior_init(int* box, int D, int W, int H) {
+  for (int k = threadIdx.x; k < D; k += blockDim.x) {
     box[k] = H;
     box[D + k] = -1;
     box[2 * D + k] = W;
@@ -59,9 +59,10 @@ __global__ void k_prior_init(int* box, int D, int W, int H, unsigned long long* 
 }
 
 // One CTA per image row: the row's intervals in shared memory, then the planes'
-// bounding boxes.  Pixels with a non-finite prior want no plane.
-__global__ void k_prior_mask(const float* __restrict__ prior, int W, int H, int D, int dmin,
-                             int dmax, int band, int16_t* mx0, int16_t* mx1, int* box) {
+// bounding boxes.  Pixels with a non-finite prior want no plane.  mx: per row and plane
+// the interval, first | last << 16 (empty: W | -1), Dpad planes a row.
+__global__ void k_prior_mask(const float* __restrict__ prior, int W, int H, int D, int Dpad,
+                             int dmin, int dmax, int band, uint32_t* mx, int* box) {
   extern __shared__ int sm[];
   int* r0 = sm;
   int* r1 = sm + D;
@@ -83,10 +84,9 @@ __global__ void k_prior_mask(const float* __restrict__ prior, int W, int H, int 
     }
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < D; k += blockDim.x) {
-    const int a = r0[k], b = r1[k];
-    mx0[size_t(y) * D + k] = int16_t(a);
-    mx1[size_t(y) * D + k] = int16_t(b);
+  for (int k = threadIdx.x; k < Dpad; k += blockDim.x) {
+    const int a = k < D ? r0[k] : W, b = k < D ? r1[k] : -1;
+    mx[size_t(y) * Dpad + k] = pack2(a, b);
     if (b < a) continue;
     atomicMin(&box[k], y);
     atomicMax(&box[D + k], y);
@@ -95,108 +95,255 @@ __global__ void k_prior_mask(const float* __restrict__ prior, int W, int H, int 
   }
 }
 
-__device__ __forceinline__ int32_t score_at(const DevCfg& c, const DevPair& P, int y, int x,
-                                            int d) {
-  const uint64_t wl = P.cwL[size_t(y) * P.cpitch + P.lpad + x];
-  const uint64_t wr = P.cwR[size_t(y) * P.cpitch + x - d];
-  int h;
-  if (c.packed) {
-    const uint32_t lo = uint32_t(wl) ^ uint32_t(wr);
-    const uint32_t hi = uint32_t(wl >> 32) ^ uint32_t(wr >> 32);
-    h = __popc(lo) + __popc(hi & 0xFFFFu);
-  } else {
-    h = __popcll(wl ^ wr);
+// A plane's extent along one direction as a filter coefficient rule.
+struct Span {
+  int lo = 1 << 28, n = 0;               // first position, positions after it
+  __device__ __forceinline__ int last() const { return lo + n; }
+  // forward step at p, with coefficient a inside
+  __device__ __forceinline__ int down(int p, int a) const {
+    return unsigned(p - lo - 1) < unsigned(n) ? a : (p == lo ? 0 : kHold);
   }
-  const int a = abs(int(P.L[size_t(y) * P.W + x]) - int(P.R[size_t(y) * P.W + x - d]));
-  return (int32_t(c.tbl[h]) * (1024 - c.wq) + int32_t(c.adt[a]) * c.wq) >> 10;
-}
+  // backward step at p (its coefficient is position p + 1's); the last position holds the
+  // forward value
+  __device__ __forceinline__ int up(int p, int a) const {
+    return unsigned(p - lo) < unsigned(n) ? a : kHold;
+  }
+};
 
-__device__ __forceinline__ int32_t rf(int32_t c, int32_t f, int32_t a) {
-  return c + ((a * (f - c) + (1 << 14)) >> 15);
-}
+__device__ __forceinline__ int warp_min(int v) { return __reduce_min_sync(0xffffffffu, v); }
+__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 
-// Horizontal passes over each needed plane's rectangle: thread = (row, plane).
-__global__ void k_prior_rows(DevCfg cfg, DevPair P, const int* __restrict__ box) {
-  const int D = P.D, W = P.W, H = P.H, Dpad = P.Dpad;
-  const int y = blockIdx.y;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= D) return;
-  const int d = cfg.dmin + k;
-  Rect r;
-  if (!plane_rect(box, D, k, W, H, cfg.hw, cfg.hh, d, &r) || y < r.ylo || y >= r.yhi) return;
-  int16_t* v = P.vol + size_t(y) * W * Dpad + k;
-  const uint16_t* ax = P.ax + size_t(y) * P.apitch + P.lpad;
-  int32_t f = score_at(cfg, P, y, r.xlo, d);
-  v[size_t(r.xlo) * Dpad] = int16_t(f);
-  for (int x = r.xlo + 1; x < r.xhi; ++x) {
-    f = rf(score_at(cfg, P, y, x, d), f, ax[x]);
-    v[size_t(x) * Dpad] = int16_t(f);
+// Horizontal passes over each needed plane's rectangle: CTA = row, thread = two planes.
+// The forward results go to the volume and come back eight words ahead.
+template <int TS>
+__global__ void __launch_bounds__(128) k_prior_rows(DevCfg cfg, DevPair P,
+                                                    const int* __restrict__ box) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int D = P.D, W = P.W, H = P.H, XS = P.Dpad / 2;
+  const int y = blockIdx.x, tid = threadIdx.x;
+  Span s0, s1;
+  for (int j = 0; j < 2; ++j) {
+    const int k = 2 * tid + j;
+    Rect r;
+    if (k >= D || !plane_rect(box, D, k, W, H, cfg.hw, cfg.hh, cfg.dmin + k, &r) || y < r.ylo ||
+        y >= r.yhi)
+      continue;
+    Span& sp = j ? s1 : s0;
+    sp.lo = r.xlo;
+    sp.n = r.xhi - r.xlo - 1;
   }
-  for (int x = r.xhi - 2; x >= r.xlo; --x) {
-    f = rf(v[size_t(x) * Dpad], f, ax[x + 1]);
-    v[size_t(x) * Dpad] = int16_t(f);
+  const int lo = min(s0.lo, s1.lo), hi = max(s0.n ? s0.last() : -1, s1.n ? s1.last() : -1);
+  if (!__syncthreads_or(hi >= 0)) return;
+  uint64_t* sL = reinterpret_cast<uint64_t*>(smem);
+  uint64_t* sR = sL + W;
+  uint8_t* tab = reinterpret_cast<uint8_t*>(sR + W);
+  uint16_t* sax = reinterpret_cast<uint16_t*>(tab + ScoreTable<TS, 1>::bytes());
+  for (int x = tid; x < W; x += blockDim.x) {
+    sL[x] = P.cwL[size_t(y) * P.cpitch + P.lpad + x];
+    sR[x] = P.cwR[size_t(y) * P.cpitch + x];
+    sax[x] = P.ax[size_t(y) * P.apitch + P.lpad + x];
   }
-}
-
-__device__ __forceinline__ void top2_insert(unsigned long long* p, uint32_t key, int* err) {
-  unsigned long long old = *reinterpret_cast<volatile unsigned long long*>(p);
-  for (int i = 0; i < kCasLimit; ++i) {
-    const uint32_t k0 = uint32_t(old >> 32), k1 = uint32_t(old);
-    if (key <= k1) return;                               // keys are unique per plane
-    const unsigned long long nv =
-        key > k0 ? (static_cast<unsigned long long>(key) << 32) | k0
-                 : (static_cast<unsigned long long>(k0) << 32) | key;
-    const unsigned long long seen = atomicCAS(p, old, nv);
-    if (seen == old) return;
-    old = seen;
+  fill_scores<TS>(cfg, tab);
+  __syncthreads();
+  const int xs = warp_min(lo), xe = warp_max(hi);       // the warp's planes
+  if (xe < 0) return;
+  // inside every needed plane's rectangle the coefficient is the image's (what the other
+  // planes hold is not looked at)
+  const int xi = warp_max(max(s0.n ? s0.lo : -1, s1.n ? s1.lo : -1));
+  const int xj = warp_min(min(s0.n ? s0.last() : 1 << 28, s1.n ? s1.last() : 1 << 28));
+  const int d0 = cfg.dmin + 2 * tid;
+  uint32_t* out = reinterpret_cast<uint32_t*>(P.vol) + size_t(y) * W * XS + tid;
+  int32_t f0 = kVolBias, f1 = kVolBias;
+  // (a lane before its own rectangle reads a clamped right word that nothing looks at)
+  uint64_t rprev = sR[max(xs - 1 - d0, 0)];
+#pragma unroll 4
+  for (int x = xs; x <= xe; ++x) {
+    const uint64_t lw = sL[x], rw = sR[max(x - d0, 0)];
+    const int a = sax[x];
+    const int32_t c0 = graded<true, TS, 1>(lw, rw, tab, nullptr, nullptr, 0, 0);
+    const int32_t c1 = graded<true, TS, 1>(lw, rprev, tab, nullptr, nullptr, 0, 0);
+    rprev = rw;
+    int a0 = a, a1 = a;
+    if (x <= xi || x > xj) { a0 = s0.down(x, a); a1 = s1.down(x, a); }
+    f0 = rf_step(c0, f0, a0);
+    f1 = rf_step(c1, f1, a1);
+    if (x >= lo && x <= hi) out[size_t(x) * XS] = pack2(f0, f1);
   }
-  if (err) atomicExch(err, 2);
-}
-
-// Vertical passes and the masked insert: thread = (column, plane).
-__global__ void k_prior_cols(DevCfg cfg, DevPair P, const int* __restrict__ box,
-                             const int16_t* __restrict__ mx0, const int16_t* __restrict__ mx1,
-                             unsigned long long* top2, int* err) {
-  const int D = P.D, W = P.W, H = P.H, Dpad = P.Dpad;
-  const int x = blockIdx.y;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= D) return;
-  const int d = cfg.dmin + k;
-  Rect r;
-  if (!plane_rect(box, D, k, W, H, cfg.hw, cfg.hh, d, &r) || x < r.xlo || x >= r.xhi) return;
-  int16_t* col = P.vol + size_t(x) * Dpad + k;
-  const size_t st = size_t(W) * Dpad;
-  int32_t f = col[size_t(r.ylo) * st];
-  for (int y = r.ylo + 1; y < r.yhi; ++y) {
-    f = rf(col[size_t(y) * st], f, P.ay[size_t(y) * W + x]);
-    col[size_t(y) * st] = int16_t(f);
-  }
-  const int iy0 = max(r.ylo, r.pylo), iy1 = min(r.yhi, r.pyhi + 1);
-  const uint32_t kk = uint32_t(255 - k);
-  auto insert = [&](int y, int32_t v) {
-    if (y < iy0 || y >= iy1) return;
-    const int xa = max(r.xlo, int(mx0[size_t(y) * D + k]));
-    const int xb = min(r.xhi, int(mx1[size_t(y) * D + k]) + 1);
-    if (x < xa || x >= xb) return;
-    const uint32_t key = (uint32_t(v + 32768) << 8) | kk;
-    top2_insert(top2 + size_t(y) * W + x, key, err);
-    if (P.rkey) atomicMax(P.rkey + size_t(y) * W + x - d, key);
+  // backward, eight words ahead
+  constexpr int PF = 8;
+  uint32_t cur[PF], nxt[PF];
+  auto fetch = [&](int x, uint32_t (&w)[PF]) {
+#pragma unroll
+    for (int i = 0; i < PF; ++i) w[i] = __ldcg(out + size_t(max(x - i, xs)) * XS);
   };
-  insert(r.yhi - 1, f);                                  // the last row: forward value
-  for (int y = r.yhi - 2; y >= r.ylo; --y) {
-    f = rf(col[size_t(y) * st], f, P.ay[size_t(y + 1) * W + x]);
-    insert(y, f);
+  fetch(xe - 1, cur);
+  for (int x = xe - 1; x >= xs; x -= PF) {
+    fetch(x - PF, nxt);
+#pragma unroll
+    for (int i = 0; i < PF; ++i) {
+      const int p = x - i;
+      if (p < xs) break;
+      const int a = sax[p + 1];
+      int a0 = a, a1 = a;
+      if (p < xi || p >= xj) { a0 = s0.up(p, a); a1 = s1.up(p, a); }
+      f0 = rf_step(int32_t(cur[i] & 0xFFFFu), f0, a0);
+      f1 = rf_step(int32_t(cur[i] >> 16), f1, a1);
+      if (p >= lo && p <= hi) out[size_t(p) * XS] = pack2(f0, f1);
+    }
+#pragma unroll
+    for (int i = 0; i < PF; ++i) cur[i] = nxt[i];
   }
 }
 
-__global__ void k_prior_keys(DevPair P, const unsigned long long* top2) {
-  const long long WH = (long long)P.W * P.H;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < WH;
-       i += (long long)gridDim.x * blockDim.x) {
-    const unsigned long long t = top2[i];
-    P.key0[i] = uint32_t(t >> 32);
-    P.key1[i] = uint32_t(t);
-    P.nb[i] = 0x80008000u;                               // no sub-pixel neighbours
+// Vertical passes and the masked top-2: TPC lanes a column, KT planes a lane: four planes
+// up to Dpad 128 (a warp per column: the most warps for one pair), else eight.
+template <int KT, int TPC>
+__global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
+                                                    const int* __restrict__ box,
+                                                    const uint32_t* __restrict__ mx) {
+  constexpr int KW = KT / 2, PF = KT == 4 ? 8 : 4;     // words a lane and row, rows ahead
+  const int D = P.D, W = P.W, H = P.H, Dpad = P.Dpad;
+  const int sub = threadIdx.x % TPC, k0 = sub * KT;
+  const int x = cfg.hw + cfg.dmin + blockIdx.x * (128 / TPC) + threadIdx.x / TPC;
+  Span sp[KT];
+  uint32_t on = 0;                       // planes needed in this column
+  int lo = 1 << 28, hi = -1, in_lo = -1, in_hi = 1 << 28;
+#pragma unroll
+  for (int i = 0; i < KT; ++i) {
+    Rect r;
+    if (k0 + i >= D || !plane_rect(box, D, k0 + i, W, H, cfg.hw, cfg.hh, cfg.dmin + k0 + i, &r) ||
+        x < r.xlo || x >= r.xhi)
+      continue;
+    sp[i].lo = r.ylo;
+    sp[i].n = r.yhi - r.ylo - 1;
+    lo = min(lo, r.ylo);
+    hi = max(hi, r.yhi - 1);
+    on |= 1u << i;
+    in_lo = max(in_lo, r.ylo);
+    in_hi = min(in_hi, r.yhi - 1);
+  }
+  const int ys = warp_min(lo), ye = warp_max(hi);       // the warp's planes
+  if (ye < 0) return;
+  const int yi = warp_max(in_lo), yj = warp_min(in_hi);   // inside all of them between
+  const int xc = min(x, W - 1), kc = min(k0, Dpad - KT);   // any address for idle lanes
+  const size_t st = size_t(W) * Dpad / 2;
+  uint32_t* col = reinterpret_cast<uint32_t*>(P.vol) + (size_t(xc) * Dpad + kc) / 2;
+  const uint16_t* ay = P.ay + xc;
+  int32_t f[KT];
+#pragma unroll
+  for (int i = 0; i < KT; ++i) f[i] = kVolBias;
+  auto load = [&](int y, uint32_t (&w)[KW]) {
+    const uint32_t* g = col + size_t(y) * st;
+    if constexpr (KW == 2) {
+      const uint2 v = __ldcg(reinterpret_cast<const uint2*>(g));
+      w[0] = v.x; w[1] = v.y;
+    } else {
+      const uint4 v = __ldcg(reinterpret_cast<const uint4*>(g));
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    }
+  };
+  uint32_t ring[PF][KW];
+  int ring_a[PF];
+#pragma unroll
+  for (int j = 0; j < PF; ++j) {
+    load(min(ys + j, ye), ring[j]);
+    ring_a[j] = ay[size_t(min(ys + j, ye)) * W];
+  }
+  for (int y0 = ys; y0 <= ye; y0 += PF) {
+#pragma unroll
+    for (int j = 0; j < PF; ++j) {
+      const int y = y0 + j;
+      uint32_t c[KW];
+#pragma unroll
+      for (int i = 0; i < KW; ++i) c[i] = ring[j][i];
+      const int a = ring_a[j];
+      load(min(y + PF, ye), ring[j]);
+      ring_a[j] = ay[size_t(min(y + PF, ye)) * W];
+      if (y > ye) continue;
+      int co[KT];
+#pragma unroll
+      for (int i = 0; i < KT; ++i) co[i] = a;
+      if (y <= yi || y > yj) {
+#pragma unroll
+        for (int i = 0; i < KT; ++i) co[i] = sp[i].down(y, a);
+      }
+#pragma unroll
+      for (int i = 0; i < KT; ++i)
+        f[i] = rf_step(int32_t(i & 1 ? c[i / 2] >> 16 : c[i / 2] & 0xFFFFu), f[i], co[i]);
+      if (y >= lo && y <= hi) {
+        uint32_t* g = col + size_t(y) * st;
+        if constexpr (KW == 2)
+          *reinterpret_cast<uint2*>(g) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
+        else
+          *reinterpret_cast<uint4*>(g) = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]),
+                                                    pack2(f[4], f[5]), pack2(f[6], f[7]));
+      }
+    }
+  }
+  // backward and the insert; a row's intervals come with its words
+  uint4 ring_m[PF][KT / 4];
+  auto load_m = [&](int y, uint4 (&m)[KT / 4]) {
+#pragma unroll
+    for (int i = 0; i < KT / 4; ++i)
+      m[i] = reinterpret_cast<const uint4*>(mx + size_t(y) * Dpad + kc)[i];
+  };
+#pragma unroll
+  for (int j = 0; j < PF; ++j) {
+    const int y = max(ye - j, ys);
+    load(y, ring[j]);
+    load_m(y, ring_m[j]);
+    ring_a[j] = ay[size_t(min(y + 1, H - 1)) * W];
+  }
+  for (int y0 = ye; y0 >= ys; y0 -= PF) {
+#pragma unroll
+    for (int j = 0; j < PF; ++j) {
+      const int y = y0 - j;
+      uint32_t c[KW];
+      uint4 m[KT / 4];
+#pragma unroll
+      for (int i = 0; i < KW; ++i) c[i] = ring[j][i];
+#pragma unroll
+      for (int i = 0; i < KT / 4; ++i) m[i] = ring_m[j][i];
+      const int a = ring_a[j], yn = max(y - PF, ys);
+      load(yn, ring[j]);
+      load_m(yn, ring_m[j]);
+      ring_a[j] = ay[size_t(min(yn + 1, H - 1)) * W];
+      if (y < ys) continue;
+      int co[KT];
+#pragma unroll
+      for (int i = 0; i < KT; ++i) co[i] = a;
+      if (y < yi || y >= yj) {
+#pragma unroll
+        for (int i = 0; i < KT; ++i) co[i] = sp[i].up(y, a);
+      }
+      uint32_t p0 = 0, p1 = 0;
+#pragma unroll
+      for (int i = 0; i < KT; ++i) {
+        f[i] = rf_step(int32_t(i & 1 ? c[i / 2] >> 16 : c[i / 2] & 0xFFFFu), f[i], co[i]);
+        const uint4 q = m[i / 4];
+        const uint32_t w = i % 4 == 0 ? q.x : i % 4 == 1 ? q.y : i % 4 == 2 ? q.z : q.w;
+        // (a needed plane's rows with an interval lie in its rectangle)
+        const bool in = on >> i & 1 && x >= int(int16_t(w & 0xFFFFu)) &&
+                        x <= (int32_t(w) >> 16);
+        const uint32_t key = in ? (uint32_t(f[i]) << 8) | uint32_t(255 - k0 - i) : 0u;
+        const uint32_t l = min(p0, key);
+        p0 = max(p0, key);
+        p1 = max(p1, l);
+        if (P.rkey && in) atomicMax(P.rkey + size_t(y) * W + x - cfg.dmin - k0 - i, key);
+      }
+      if (!__any_sync(0xffffffffu, p0 != 0)) continue;
+#pragma unroll
+      for (int o = 1; o < TPC; o <<= 1) {
+        const uint32_t o0 = __shfl_xor_sync(0xffffffffu, p0, o), o1 = __shfl_xor_sync(0xffffffffu, p1, o);
+        const uint32_t l = min(p0, o0);
+        p0 = max(p0, o0);
+        p1 = max(max(p1, o1), l);
+      }
+      if (sub == 0 && p0) {
+        P.key0[size_t(y) * W + x] = p0;
+        P.key1[size_t(y) * W + x] = p1;
+      }
+    }
   }
 }
 
@@ -204,29 +351,38 @@ __global__ void k_prior_keys(DevPair P, const unsigned long long* top2) {
 
 size_t prior_ws_bytes(int W, int H, int D) {
   auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
-  return 2 * up(size_t(H) * D * 2) + up(size_t(D) * 16) + up(size_t(W) * H * 8);
+  return up(size_t(H) * ((D + 63) & ~63) * 4) + up(size_t(D) * 16);
 }
 
 cudaError_t launch_prior(const DevCfg& cfg, const Batch& b, const float* prior, int band,
                          void* ws, cudaStream_t s) {
   const DevPair& P = b.p[0];
-  const int W = P.W, H = P.H, D = P.D;
+  const int W = P.W, H = P.H, D = P.D, Dpad = P.Dpad;
   auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
-  uint8_t* p = static_cast<uint8_t*>(ws);
-  int16_t* mx0 = reinterpret_cast<int16_t*>(p);                 p += up(size_t(H) * D * 2);
-  int16_t* mx1 = reinterpret_cast<int16_t*>(p);                 p += up(size_t(H) * D * 2);
-  int* box = reinterpret_cast<int*>(p);                         p += up(size_t(D) * 16);
-  unsigned long long* top2 = reinterpret_cast<unsigned long long*>(p);
-  const long long WH = (long long)W * H;
-  k_prior_init<<<int(std::min<long long>((WH + 255) / 256, 1184)), 256, 0, s>>>(box, D, W, H,
-                                                                               top2, WH);
-  k_prior_mask<<<H, 256, size_t(2) * D * sizeof(int), s>>>(prior, W, H, D, cfg.dmin,
-                                                           cfg.dmin + D - 1, band, mx0, mx1,
-                                                           box);
-  const int kb = (D + 127) / 128;
-  k_prior_rows<<<dim3(kb, H), 128, 0, s>>>(cfg, P, box);
-  k_prior_cols<<<dim3(kb, W), 128, 0, s>>>(cfg, P, box, mx0, mx1, top2, b.err);
-  k_prior_keys<<<int(std::min<long long>((WH + 255) / 256, 1184)), 256, 0, s>>>(P, top2);
+  uint32_t* mx = static_cast<uint32_t*>(ws);
+  int* box = reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + up(size_t(H) * Dpad * 4));
+  // no candidate where no plane is inserted; sub-pixel neighbours are never looked at
+  cudaError_t e = cudaMemsetAsync(P.key0, 0, size_t(W) * H * 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(P.key1, 0, size_t(W) * H * 4, s);
+  if (e != cudaSuccess) return e;
+  k_prior_init<<<1, 256, 0, s>>>(box, D, W, H);
+  k_prior_mask<<<H, 256, size_t(2) * D * sizeof(int), s>>>(prior, W, H, D, Dpad, cfg.dmin,
+                                                           cfg.dmin + D - 1, band, mx, box);
+  auto rows = [&](auto kern, size_t table) -> cudaError_t {
+    const size_t sm = size_t(W) * 18 + table;
+    const cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    if (e2 != cudaSuccess) return e2;
+    kern<<<H, Dpad / 2, sm, s>>>(cfg, P, box);
+    return cudaGetLastError();
+  };
+  e = cfg.trunc < 16 ? rows(k_prior_rows<16>, ScoreTable<16, 1>::bytes())
+                     : rows(k_prior_rows<256>, ScoreTable<256, 1>::bytes());
+  const int ncols = W - 2 * cfg.hw - cfg.dmin;
+  if (e != cudaSuccess || ncols <= 0) return e;
+  auto grid = [&](int tpc) { return (ncols + 128 / tpc - 1) / (128 / tpc); };
+  if (Dpad == 64) k_prior_cols<4, 16><<<grid(16), 128, 0, s>>>(cfg, P, box, mx);
+  else if (Dpad == 128) k_prior_cols<4, 32><<<grid(32), 128, 0, s>>>(cfg, P, box, mx);
+  else k_prior_cols<8, 32><<<grid(32), 128, 0, s>>>(cfg, P, box, mx);
   return cudaGetLastError();
 }
 
