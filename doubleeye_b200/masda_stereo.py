@@ -148,6 +148,14 @@ def _seg_max_excluding(vals, idx, n):
     return _np(out[:E])
 
 
+def _assignment(a) -> dict:
+    """left -> right of an assignment array (-1: none), ascending.  Whole-array
+    conversions: with int() per entry the dict of a 450x375 map (147 k entries) took 21 ms
+    of a 28 ms solve, this 9 ms."""
+    left = np.flatnonzero(a >= 0)
+    return dict(zip(left.tolist(), a[left].tolist()))
+
+
 def _solve(ei, ej, se, m, n, lam, gam, iters, damping, eps, want_belief=False):
     torch = _torch()
     E = int(se.numel())
@@ -165,8 +173,7 @@ def _solve(ei, ej, se, m, n, lam, gam, iters, damping, eps, want_belief=False):
                                    else None, ws.data_ptr(), need.value, _stream()))
     k = int(nh.item())
     a = _np(assign[:m])
-    out = {int(i): int(j) for i, j in zip(np.nonzero(a >= 0)[0], a[a >= 0])}
-    return out, _np(hist[:k]), belief
+    return _assignment(a), _np(hist[:k]), belief
 
 
 def masda_sparse(ei, ej, se, m, n, lam=-0.1, gam=-0.1, iters=30, damping=0.4, eps=1e-5):
@@ -218,4 +225,4 @@ def decide(S, belief, lam):
     else:
         assign.fill_(-1)
     a = _np(assign[:m])
-    return {int(i): int(j) for i, j in zip(np.nonzero(a >= 0)[0], a[a >= 0])}
+    return _assignment(a)
