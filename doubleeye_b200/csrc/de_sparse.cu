@@ -474,8 +474,6 @@ __global__ void __launch_bounds__(1024) k_det_emit(int cells, int keep, DetWs d,
 struct MatchWs {
   int* cnt;          // [nl + 1] candidates per left point, then row offsets
   int* slot_j;       // [nl * maxc]
-  float* slot_s;     // [nl * maxc]
-  int* order;        // [nr] right points in (y, index) order
   int* ei;           // [E] edge lists in the reference's edge order
   int* ej;
   float* es;
@@ -501,7 +499,7 @@ __host__ __device__ inline size_t up256(size_t b) { return (b + 255) & ~size_t(2
 size_t match_ws_bytes(int nl, int nr, int maxc) {
   const size_t E = size_t(nl) * maxc;
   const size_t L = size_t(nl) + 1, R = size_t(nr) + 1;
-  return up256(L * 4) + up256(E * 4) * 2 + up256(R * 4) + up256(E * 4) * 6 + up256(R * 4) * 2 +
+  return up256(L * 4) + up256(E * 4) * 7 + up256(R * 4) * 2 +
          up256(E * 4) + up256(L * 4) + up256(R * 4) + up256(L * 4) + up256(L) + up256(R) +
          up256(L * 4) + up256(R * 4) + up256(L * 4) + up256(L * 4);
 }
@@ -514,8 +512,6 @@ MatchWs carve_match(void* ws, int nl, int nr, int maxc) {
   MatchWs m;
   m.cnt = reinterpret_cast<int*>(take(L * 4));
   m.slot_j = reinterpret_cast<int*>(take(E * 4));
-  m.slot_s = reinterpret_cast<float*>(take(E * 4));
-  m.order = reinterpret_cast<int*>(take(R * 4));
   m.ei = reinterpret_cast<int*>(take(E * 4));
   m.ej = reinterpret_cast<int*>(take(E * 4));
   m.es = reinterpret_cast<float*>(take(E * 4));
@@ -558,6 +554,9 @@ struct MatchArgs {
 __device__ __forceinline__ uint32_t ord_f32(float v) {   // order-preserving bits
   const uint32_t b = __float_as_uint(v);
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float unord_f32(uint32_t b) {
+  return __uint_as_float((b & 0x80000000u) ? b & 0x7fffffffu : ~b);
 }
 
 // pair_score, core/src/match.cpp:298-332: descriptor agreement minus the y-residual
@@ -626,6 +625,16 @@ __device__ float cta_max(float v, float* red) {
   return r;
 }
 
+// The CTA's greatest of values >= 0 (whose bits order as they do).
+__device__ float cta_max_pos(float v, int* red) {
+  const int w = __reduce_max_sync(0xffffffffu, __float_as_int(v));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = w;
+  __syncthreads();
+  const int r = __reduce_max_sync(0xffffffffu, red[threadIdx.x & 31]);   // 32 warps
+  __syncthreads();
+  return __int_as_float(r);
+}
+
 __device__ int cta_or(int v, int* red) {
   v = __any_sync(0xffffffffu, v);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
@@ -636,110 +645,122 @@ __device__ int cta_or(int v, int* red) {
   return r;
 }
 
-__global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, MatchWs m) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  uint64_t* keys = reinterpret_cast<uint64_t*>(smem);
-  __shared__ int warp_sums[32];
-  __shared__ float redf[32];
-  __shared__ int redi[32];
-  __shared__ int s_nacc;
-  const int tid = threadIdx.x, NT = blockDim.x;
-  const int nl = a.nl_dev ? max(0, min(a.nl_cap, *a.nl_dev)) : a.nl_cap;
-  const int nr = a.nr_dev ? max(0, min(a.nr_cap, *a.nr_dev)) : a.nr_cap;
-  const int maxc = a.maxc;
-
-  // --- right points in y order (ties by index) -------------------------------------
-  int N = 1;
-  while (N < nr) N <<= 1;
-  for (int i = tid; i < N; i += NT)
-    keys[i] = (i < nr) ? (uint64_t(ord_f32(a.kr[i].y)) << 32) | uint32_t(i) : ~0ull;
+// Sorts keys[0..n) (distinct; their high words the order-preserving bits of a float) with
+// tmp and bins as scratch: bins on a linear map of the floats, then each key's rank among
+// its bin's.  Returns false, with keys as they were, where the floats or their spread do
+// not suit (the bitonic sort takes those).  2430 keypoint rows: 7 us against 52.
+constexpr int kSortBins = 4096, kSortBinMax = 64;
+__device__ bool cta_bin_sort(uint64_t* keys, uint64_t* tmp, int* bins, int n, int* warp_sums,
+                             float* red) {
+  float lo = 3e38f, hi = -3e38f;
+  int odd = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const float y = unord_f32(uint32_t(keys[i] >> 32));
+    odd |= !isfinite(y);
+    lo = fminf(lo, y);
+    hi = fmaxf(hi, y);
+  }
+  hi = cta_max(hi, red);
+  lo = -cta_max(-lo, red);
+  const float scale = float(kSortBins - 1) / (hi - lo);
+  if (__syncthreads_or(odd || !isfinite(scale))) return false;
+  auto bin = [&](uint64_t k) {           // monotone: so are the subtraction and the product
+    return min(kSortBins - 1, int((unord_f32(uint32_t(k >> 32)) - lo) * scale));
+  };
+  for (int i = threadIdx.x; i < kSortBins; i += blockDim.x) bins[i] = 0;
   __syncthreads();
-  cta_bitonic(keys, N, [](uint64_t x, uint64_t y) { return x < y; });
-  for (int i = tid; i < nr; i += NT) m.order[i] = int(keys[i] & 0xffffffffu);
-  __syncthreads();
-
-  // --- candidate rows (build_candidates) --------------------------------------------
-  for (int i = tid; i < nl; i += NT) {
-    const de_keypoint l = a.kl[i];
-    const uint32_t klo = ord_f32(l.y - a.max_dy), khi = ord_f32(l.y + a.max_dy);
-    int lo = 0, hi = nr;
-    {
-      int p = 0, q = nr;
-      while (p < q) {
-        const int md = (p + q) >> 1;
-        if (uint32_t(keys[md] >> 32) < klo) p = md + 1; else q = md;
-      }
-      lo = p;
-      q = nr;
-      while (p < q) {
-        const int md = (p + q) >> 1;
-        if (!(khi < uint32_t(keys[md] >> 32))) p = md + 1; else q = md;
-      }
-      hi = p;
-    }
-    int ns = 0;
-    for (int p = lo; p < hi; ++p) {
-      const float d = l.x - a.kr[int(keys[p] & 0xffffffffu)].x;
-      ns += (d < a.min_disp || d > a.max_disp) ? 0 : 1;
-    }
-    const uint64_t dli = a.dl[i];
-    int* sj = m.slot_j + size_t(i) * maxc;
-    float* ss = m.slot_s + size_t(i) * maxc;
-    if (ns <= maxc) {
-      int k = 0;
-      for (int p = lo; p < hi; ++p) {
-        const int j = int(keys[p] & 0xffffffffu);
-        const de_keypoint r = a.kr[j];
-        const float d = l.x - r.x;
-        if (d < a.min_disp || d > a.max_disp) continue;
-        sj[k] = j;
-        ss[k] = pair_score(l, r, dli, a.dr[j], a, i);
-        ++k;
-      }
-    } else {                  // best maxc by score, in score order (ties: band order)
-      for (int p = lo; p < hi; ++p) {
-        const int j = int(keys[p] & 0xffffffffu);
-        const de_keypoint r = a.kr[j];
-        const float d = l.x - r.x;
-        if (d < a.min_disp || d > a.max_disp) continue;
-        const float s = pair_score(l, r, dli, a.dr[j], a, i);
-        int rank = 0;
-        for (int q = lo; q < hi && rank < maxc; ++q) {
-          const int jq = int(keys[q] & 0xffffffffu);
-          const de_keypoint rq = a.kr[jq];
-          const float dq = l.x - rq.x;
-          if (dq < a.min_disp || dq > a.max_disp) continue;
-          const float sq = pair_score(l, rq, dli, a.dr[jq], a, i);
-          rank += (sq > s || (sq == s && q < p)) ? 1 : 0;
-        }
-        if (rank < maxc) {
-          sj[rank] = j;
-          ss[rank] = s;
-        }
-      }
-    }
-    m.cnt[i] = min(ns, maxc);
+  int most = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) most = max(most, atomicAdd(&bins[bin(keys[i])], 1));
+  if (__syncthreads_or(most >= kSortBinMax)) return false;
+  cta_excl_scan<1024>(bins, kSortBins, warp_sums);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) tmp[atomicAdd(&bins[bin(keys[i])], 1)] = keys[i];
+  __syncthreads();                       // bins[b] is now the end of bin b
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const uint64_t k = tmp[i];
+    const int b = bin(k), first = b ? bins[b - 1] : 0, end = bins[b];
+    int rank = first;
+    for (int q = first; q < end; ++q) rank += tmp[q] < k;
+    keys[rank] = k;
   }
   __syncthreads();
-  const int E = cta_excl_scan<1024>(m.cnt, nl, warp_sums);
+  return true;
+}
+
+// Points 0..n in order of degree (ptr[i + 1] - ptr[i]), so that the lanes of a warp walk
+// edge lists of one length.  bins: 65 ints of scratch.
+__device__ void by_degree(const int* ptr, int n, uint16_t* perm, int* bins) {
+  for (int i = threadIdx.x; i < 65; i += blockDim.x) bins[i] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&bins[min(63, ptr[i + 1] - ptr[i])], 1);
+  __syncthreads();
+  if (threadIdx.x < 32) {                // exclusive scan, two bins a lane
+    const int d = 2 * threadIdx.x, c0 = bins[d], c = c0 + bins[d + 1];
+    int v = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (int(threadIdx.x) >= o) v += u;
+    }
+    bins[d] = v - c;
+    bins[d + 1] = v - c + c0;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    perm[atomicAdd(&bins[min(63, ptr[i + 1] - ptr[i])], 1)] = uint16_t(i);
+  __syncthreads();
+}
+
+// From the candidate lists on: edge lists, sweeps, beliefs, decision.  All of it walks edge
+// lists with dependent loads, so with NEAR (a few thousand edges) every array is in
+// shared memory, where arrays that are never live together share storage; else the
+// caller's workspace holds them.
+template <bool NEAR>
+__device__ __forceinline__ void match_tail(const MatchArgs& a, const MatchWs& ws, uint8_t* smem,
+                                           int nl, int nr, int E, int* warp_sums, int* redi,
+                                           int* s_deg, int& s_nacc) {
+  const int tid = threadIdx.x, NT = blockDim.x;
+  MatchWs m = ws;
+  uint16_t *lperm = nullptr, *rperm = nullptr;
+  int* sidx = reinterpret_cast<int*>(smem);             // the last sort's places
+  if constexpr (NEAR) {
+    int N2 = 1;
+    while (N2 < min(nl, nr)) N2 <<= 1;
+    size_t o = size_t(N2) * 4;
+    auto take = [&](size_t b) { const size_t q = o; o += (b + 3) & ~size_t(3); return smem + q; };
+    m.cnt = reinterpret_cast<int*>(take(size_t(nl + 1) * 4));
+    m.cstart = reinterpret_cast<int*>(take(size_t(nr + 1) * 4));
+    m.cfill = m.best_col = m.cbest = reinterpret_cast<int*>(take(size_t(nr) * 4));
+    m.best_row = m.rbest = reinterpret_cast<int*>(take(size_t(nl) * 4));
+    m.margin = reinterpret_cast<float*>(take(size_t(nl) * 4));
+    m.flag = m.acc = reinterpret_cast<int*>(take(size_t(nl + 1) * 4));
+    m.ei = reinterpret_cast<int*>(take(size_t(E) * 4));
+    m.ej = reinterpret_cast<int*>(take(size_t(E) * 4));
+    m.es = reinterpret_cast<float*>(take(size_t(E) * 4));
+    m.beta = reinterpret_cast<float*>(take(size_t(E) * 4));
+    m.rho = m.belief = reinterpret_cast<float*>(take(size_t(E) * 4));
+    m.citems = reinterpret_cast<int*>(take(size_t(E) * 4));
+    lperm = reinterpret_cast<uint16_t*>(take(size_t(nl) * 2));
+    rperm = reinterpret_cast<uint16_t*>(take(size_t(nr) * 2));
+    m.rt = take(nl);
+    m.ct = take(nr);
+    for (int i = tid; i < nl; i += NT) m.cnt[i] = ws.cnt[i];
+  }
+  __syncthreads();
   if (tid == 0) m.cnt[nl] = E;
   for (int j = tid; j < nr; j += NT) {
     m.cstart[j] = 0;
     m.cfill[j] = 0;
   }
   __syncthreads();
-  for (int i = tid; i < nl; i += NT) {
-    const int b = m.cnt[i], c = m.cnt[i + 1] - b;
-    for (int k = 0; k < c; ++k) {
-      const int e = b + k;
-      const int j = m.slot_j[size_t(i) * maxc + k];
-      m.ei[e] = i;
-      m.ej[e] = j;
-      m.es[e] = m.slot_s[size_t(i) * maxc + k];
-      m.beta[e] = 0.f;
-      m.rho[e] = 0.f;
-      atomicAdd(&m.cstart[j], 1);
-    }
+  for (int i = tid; i < nl; i += NT)
+    for (int e = m.cnt[i]; e < m.cnt[i + 1]; ++e) m.ei[e] = i;
+  __syncthreads();
+  for (int e = tid; e < E; e += NT) {                   // a thread per edge: no lane waits
+    const int i = m.ei[e], j = ws.slot_j[size_t(i) * a.maxc + (e - m.cnt[i])];
+    m.ej[e] = j;
+    m.es[e] = pair_score(a.kl[i], a.kr[j], a.dl[i], a.dr[j], a, i);
+    m.beta[e] = 0.f;
+    m.rho[e] = 0.f;
+    atomicAdd(&m.cstart[j], 1);
   }
   __syncthreads();
   cta_excl_scan<1024>(m.cstart, nr, warp_sums);
@@ -752,10 +773,10 @@ __global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, MatchWs m) {
   __syncthreads();
 
   // --- damped max-sum sweeps ---------------------------------------------------------
-  // The sweeps walk each point's edges with dependent loads, so their state (row and
-  // column offsets, column items, scores, beta, rho) moves to shared memory when it
-  // fits (a few thousand edges take well under the 227 KB); the sort keys there are
-  // dead by now.  Same operations in the same order either way.
+  // Without NEAR there may still be room for the sweeps' own state (offsets, column items,
+  // scores, beta, rho).  With it a warp's lanes take points of one degree: in keypoint
+  // order each warp waits for its longest list, two edges a point on average.  Same
+  // operations in the same order within a list either way.
   const int* bcnt = m.cnt;
   const int* bcst = m.cstart;
   const int* bcit = m.citems;
@@ -763,7 +784,11 @@ __global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, MatchWs m) {
   float* bbeta = m.beta;
   float* brho = m.rho;
   const size_t bp_bytes = size_t(nl + 1 + nr + 1) * 4 + size_t(E) * 16;
-  const bool bp_smem = bp_bytes <= size_t(a.smem_bytes);
+  const bool bp_smem = !NEAR && bp_bytes <= size_t(a.smem_bytes);
+  if constexpr (NEAR) {
+    by_degree(m.cnt, nl, lperm, s_deg);
+    by_degree(m.cstart, nr, rperm, s_deg);
+  }
   if (bp_smem) {
     int* s_cnt = reinterpret_cast<int*>(smem);
     int* s_cst = s_cnt + (nl + 1);
@@ -786,46 +811,52 @@ __global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, MatchWs m) {
   const float dmp = (0.99f < d0) ? 0.99f : d0;
   float prev = 1e30f, md = 0.f;
   int it = 0, osc = 0, conv = 0;
+  // One list: out[e] from the greatest of in over the list's other edges.  Lists of one
+  // and two edges (most of them, and whole warps of them by degree) need no search.
+  auto list_pass = [&](int b, int c, auto edge, float floor, const float* in, float* out,
+                       float& loc) {
+    auto update = [&](int e, float others) {
+      const float tgt = bes[e] - fmax_ref(floor, others);
+      const float old = out[e];
+      const float upd = (1.f - dmp) * tgt + dmp * old;
+      loc = fmax_ref(loc, fabsf(upd - old));
+      out[e] = upd;
+    };
+    if (c - b <= 1) {
+      if (c > b) update(edge(b), kNegBig);
+      return;
+    }
+    if (c - b == 2) {
+      const int e0 = edge(b), e1 = edge(b + 1);
+      const float v0 = fmax_ref(kNegBig, in[e0]), v1 = fmax_ref(kNegBig, in[e1]);
+      update(e0, v1);
+      update(e1, v0);
+      return;
+    }
+    float best = kNegBig, second = kNegBig;
+    int bi = -1;
+    for (int q = b; q < c; ++q) {
+      const int e = edge(q);
+      const float v = in[e];
+      if (v > best) { second = best; best = v; bi = e; } else if (v > second) second = v;
+    }
+    for (int q = b; q < c; ++q) {
+      const int e = edge(q);
+      update(e, (e == bi) ? second : best);
+    }
+  };
   for (; it < a.iters && E > 0; ++it) {
     float loc = 0.f;
-    for (int i = tid; i < nl; i += NT) {
-      const int b = bcnt[i], c = bcnt[i + 1];
-      float best = kNegBig, second = kNegBig;
-      int bi = -1;
-      for (int e = b; e < c; ++e) {
-        const float v = bbeta[e];
-        if (v > best) { second = best; best = v; bi = e; } else if (v > second) second = v;
-      }
-      for (int e = b; e < c; ++e) {
-        const float comp = fmax_ref(a.lambda, (e == bi) ? second : best);
-        const float tgt = bes[e] - comp;
-        const float old = brho[e];
-        const float upd = (1.f - dmp) * tgt + dmp * old;
-        loc = fmax_ref(loc, fabsf(upd - old));
-        brho[e] = upd;
-      }
+    for (int t = tid; t < nl; t += NT) {
+      const int i = NEAR ? lperm[t] : t;
+      list_pass(bcnt[i], bcnt[i + 1], [](int e) { return e; }, a.lambda, bbeta, brho, loc);
     }
     __syncthreads();
-    for (int j = tid; j < nr; j += NT) {
-      const int b = bcst[j], c = bcst[j + 1];
-      float best = kNegBig, second = kNegBig;
-      int bi = -1;
-      for (int q = b; q < c; ++q) {
-        const int e = bcit[q];
-        const float v = brho[e];
-        if (v > best) { second = best; best = v; bi = e; } else if (v > second) second = v;
-      }
-      for (int q = b; q < c; ++q) {
-        const int e = bcit[q];
-        const float comp = fmax_ref(a.gamma, (e == bi) ? second : best);
-        const float tgt = bes[e] - comp;
-        const float old = bbeta[e];
-        const float upd = (1.f - dmp) * tgt + dmp * old;
-        loc = fmax_ref(loc, fabsf(upd - old));
-        bbeta[e] = upd;
-      }
+    for (int t = tid; t < nr; t += NT) {
+      const int j = NEAR ? rperm[t] : t;
+      list_pass(bcst[j], bcst[j + 1], [&](int q) { return bcit[q]; }, a.gamma, brho, bbeta, loc);
     }
-    md = cta_max(loc, redf);            // includes the barrier the next sweep needs
+    md = cta_max_pos(loc, redi);        // includes the barrier the next sweep needs
     if (md > prev) ++osc;
     prev = md;
     if (md < a.eps) {
@@ -941,7 +972,6 @@ __global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, MatchWs m) {
     __syncthreads();
   }
   const int n2 = s_nacc;
-  int* sidx = reinterpret_cast<int*>(smem);
   int N2 = 1;
   while (N2 < n2) N2 <<= 1;
   for (int k = tid; k < N2; k += NT) sidx[k] = (k < n2) ? m.acc[k] : -1;
@@ -966,6 +996,112 @@ __global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, MatchWs m) {
       *a.stats = s;
     }
   }
+}
+
+// One CTA per matching problem.  Bound by the sweeps' shared-memory latency and block
+// barriers on one SM.  848x480, 2430 keypoints a side, 5008 edges, 20 sweeps, in thousands
+// of clocks: sort 100 -> 13 (bitonic before), candidates 118 -> 30 (points read from
+// global memory, scores inside the search), edge lists 48 -> 31, sweeps 333 -> 150
+// (keypoint order), beliefs and decision 68 -> 33; the kernel 354 -> 140 us.
+__global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, const MatchWs m) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint64_t* keys = reinterpret_cast<uint64_t*>(smem);
+  __shared__ int warp_sums[32];
+  __shared__ float redf[32];
+  __shared__ int redi[32];
+  __shared__ int s_nacc;
+  __shared__ int s_deg[65];
+  const int tid = threadIdx.x, NT = blockDim.x;
+  const int nl = a.nl_dev ? max(0, min(a.nl_cap, *a.nl_dev)) : a.nl_cap;
+  const int nr = a.nr_dev ? max(0, min(a.nr_cap, *a.nr_dev)) : a.nr_cap;
+  const int maxc = a.maxc;
+
+  // --- right points in y order (ties by index) -------------------------------------
+  int N = 1;
+  while (N < nr) N <<= 1;
+  for (int i = tid; i < N; i += NT)
+    keys[i] = (i < nr) ? (uint64_t(ord_f32(a.kr[i].y)) << 32) | uint32_t(i) : ~0ull;
+  __syncthreads();
+  if (size_t(nr) * 16 + kSortBins * 4 > size_t(a.smem_bytes) ||
+      !cta_bin_sort(keys, keys + nr, reinterpret_cast<int*>(keys + 2 * size_t(nr)), nr, warp_sums,
+                    redf)) {
+    for (int i = nr + tid; i < N; i += NT) keys[i] = ~0ull;      // (scratch of the other sort)
+    __syncthreads();
+    cta_bitonic(keys, N, [](uint64_t x, uint64_t y) { return x < y; });
+  }
+
+  // --- candidate rows (build_candidates) --------------------------------------------
+  // the right points' x and descriptors in sorted order beside the keys, when they fit
+  float* sx = reinterpret_cast<float*>(keys + nr);
+  uint64_t* sd = reinterpret_cast<uint64_t*>(keys + nr + (nr + 1) / 2);
+  const bool near = size_t(nr) * 20 + 16 <= size_t(a.smem_bytes);
+  if (near)
+    for (int p = tid; p < nr; p += NT) {
+      const int j = int(keys[p] & 0xffffffffu);
+      sx[p] = a.kr[j].x;
+      sd[p] = a.dr[j];
+    }
+  __syncthreads();
+  auto right_x = [&](int p) { return near ? sx[p] : a.kr[int(keys[p] & 0xffffffffu)].x; };
+  for (int i = tid; i < nl; i += NT) {
+    const de_keypoint l = a.kl[i];
+    const uint32_t klo = ord_f32(l.y - a.max_dy), khi = ord_f32(l.y + a.max_dy);
+    int lo = 0, hi = nr;
+    {
+      int p = 0, q = nr;
+      while (p < q) {
+        const int md = (p + q) >> 1;
+        if (uint32_t(keys[md] >> 32) < klo) p = md + 1; else q = md;
+      }
+      lo = p;
+      q = nr;
+      while (p < q) {
+        const int md = (p + q) >> 1;
+        if (!(khi < uint32_t(keys[md] >> 32))) p = md + 1; else q = md;
+      }
+      hi = p;
+    }
+    const uint64_t dli = a.dl[i];
+    int* sj = m.slot_j + size_t(i) * maxc;
+    auto score = [&](int p, float x) {
+      de_keypoint r;
+      r.x = x;
+      r.y = unord_f32(uint32_t(keys[p] >> 32));
+      return pair_score(l, r, dli, near ? sd[p] : a.dr[int(keys[p] & 0xffffffffu)], a, i);
+    };
+    int ns = 0;
+    for (int p = lo; p < hi; ++p) {
+      const float x = right_x(p), d = l.x - x;
+      if (d < a.min_disp || d > a.max_disp) continue;
+      if (ns < maxc) sj[ns] = int(keys[p] & 0xffffffffu);
+      ++ns;
+    }
+    if (ns > maxc) {          // best maxc by score, in score order (ties: band order)
+      for (int p = lo; p < hi; ++p) {
+        const float x = right_x(p), d = l.x - x;
+        if (d < a.min_disp || d > a.max_disp) continue;
+        const float s = score(p, x);
+        int rank = 0;
+        for (int q = lo; q < hi && rank < maxc; ++q) {
+          const float xq = right_x(q), dq = l.x - xq;
+          if (dq < a.min_disp || dq > a.max_disp) continue;
+          const float sq = score(q, xq);
+          rank += (sq > s || (sq == s && q < p)) ? 1 : 0;
+        }
+        if (rank < maxc) sj[rank] = int(keys[p] & 0xffffffffu);
+      }
+    }
+    m.cnt[i] = min(ns, maxc);
+  }
+  __syncthreads();
+  const int E = cta_excl_scan<1024>(m.cnt, nl, warp_sums);
+  int N2 = 1;
+  while (N2 < min(nl, nr)) N2 <<= 1;
+  const size_t need = size_t(N2) * 4 + size_t(E) * 24 + size_t(nl + 1) * 20 + size_t(nr + 1) * 12 + 32;
+  if (need <= size_t(a.smem_bytes) && nl < 65536)
+    match_tail<true>(a, m, smem, nl, nr, E, warp_sums, redi, s_deg, s_nacc);
+  else
+    match_tail<false>(a, m, smem, nl, nr, E, warp_sums, redi, s_deg, s_nacc);
 }
 
 
