@@ -59,7 +59,7 @@ __device__ __forceinline__ int32_t graded(uint64_t lw, uint64_t rw, const void* 
   if (PACKED) {
     const uint32_t lh = uint32_t(lw >> 32), rh = uint32_t(rw >> 32);
     h = __popc(uint32_t(lw) ^ uint32_t(rw)) + __popc((lh ^ rh) & kCensusHiMask);
-    ad = abs((int32_t(lh) - int32_t(rh)) >> kPixShift);
+    ad = int(__usad(lh >> kPixShift, rh >> kPixShift, 0u));
   } else {
     h = __popcll(lw ^ rw);
     ad = abs(int(sLp[xl]) - int(sRp[xr]));
