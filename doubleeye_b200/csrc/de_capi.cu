@@ -345,11 +345,9 @@ void part_batch(const de::Batch& b, int parts, int k, de::Batch* out) {
 
 int g_batch_streams = 2;          // parts a batch of several pairs is run as, 1..4
 
-int run_batch(const de_cfg& c, de::Batch& b, cudaStream_t s, int max_parts, bool reg_ring,
-              bool overlapped) {
+int run_batch(const de_cfg& c, de::Batch& b, cudaStream_t s, int max_parts, bool overlapped) {
   de::DevCfg dc;
   de::make_dev_cfg(c, &dc);
-  if (reg_ring) dc.cols_async = 0;
   if (c.lrc)
     for (int i = 0; i < b.n; ++i)
       DE_CUDA(cudaMemsetAsync(b.p[i].rkey, 0, size_t(b.p[i].W) * b.p[i].H * 4, s));
@@ -479,8 +477,7 @@ int de_dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspace
 }  // extern "C"
 
 int de::dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspace,
-                  size_t ws_bytes, cudaStream_t stream, int max_parts, bool reg_ring,
-                  bool overlapped) {
+                  size_t ws_bytes, cudaStream_t stream, int max_parts, bool overlapped) {
   size_t need = 0;
   int rc = de_dense_workspace_bytes(cfg, pairs, n, &need);
   if (rc) return rc;
@@ -500,7 +497,7 @@ int de::dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspac
     for (int i = 0; i < m; ++i)
       ws += de::pair_workspace_bytes(pairs[first + i].W, pairs[first + i].H,
                                      pair_D(*cfg, pairs[first + i]), cfg->lrc != 0);
-    if ((rc = run_batch(*cfg, b, s, max_parts, reg_ring, overlapped))) return rc;
+    if ((rc = run_batch(*cfg, b, s, max_parts, overlapped))) return rc;
   }
   return DE_OK;
 }
@@ -940,21 +937,18 @@ int de_ctx_dense_batch(de_ctx* c, const de_pair* hp, int n) {
   // own stream in its own workspace slice, at a priority below the chunk before it:
   // the first chunk runs as if alone and the later ones take the SMs it leaves idle
   // (its tails, its lightly occupied kernels), so chunking costs little device
-  // efficiency.  Five chunks from 8 pairs up: small ends (n/8 pairs each) keep the
-  // exposed first upload and last download short, and three equal middle chunks
-  // finish one after another so their downloads overlap the compute behind them
-  // (16 pairs of 848x480: 2, 4, 4, 4, 2).  The first chunk is uploaded and launched
-  // before anything else is prepared.
+  // efficiency.  Up to five chunks, at least a pair each, of about 21, 25, 25, 18 and 11
+  // per cent of the pairs: the last ones small, because a download after the last
+  // compute is exposed (848x480 pairs, the plan before -> this, us a call: 3 pairs 890 ->
+  // 790, 4 1125 -> 910, 6 1555 -> 1335, 8 1650 -> 1605, 12 2390 -> 2255, 16 3105 ->
+  // 2895).  The first chunk is uploaded and launched before anything else is prepared.
   int bound[de_ctx::kChunks + 1] = {0};
   int nch = 1;
-  if (out_bytes >= (size_t(8) << 20) && n >= 8) {
-    const int e = std::max(1, n / 8), mid = n - 2 * e;
-    const int sizes[5] = {e, (mid + 2) / 3, (mid + 1) / 3, mid / 3, e};
-    nch = 5;
-    for (int k = 0; k < nch; ++k) bound[k + 1] = bound[k] + sizes[k];
-  } else if (out_bytes >= (size_t(8) << 20) && n >= 4) {
-    nch = 2;
-    bound[1] = (2 * n + 2) / 3;
+  if (out_bytes >= (size_t(8) << 20) && n >= 2) {
+    static const int kPlan[de_ctx::kChunks] = {21, 46, 71, 89, 100};
+    nch = std::min(n, int(de_ctx::kChunks));
+    for (int k = 0; k < nch; ++k)
+      bound[k + 1] = std::min(std::max((n * kPlan[k] + 50) / 100, bound[k] + 1), n - (nch - 1 - k));
   }
   bound[nch] = n;
   size_t woff[de_ctx::kChunks + 1] = {0};
@@ -975,13 +969,10 @@ int de_ctx_dense_batch(de_ctx* c, const de_pair* hp, int n) {
     for (int k = 0; k < nch; ++k) {
       cudaStream_t sk = c->cs[k];
       if (k > 0) DE_CUDA(cudaStreamWaitEvent(sk, c->ev_in[k], 0));
-      // chunks already overlap one another: each runs as one launch set, with the
-      // column kernel's ring in registers (its shared-memory ring, which frees room
-      // for a second launch set of the same batch, crowds five concurrent chunks:
-      // e2e 4990 -> 5045 pairs/s with the register ring here)
+      // chunks already overlap one another: each runs as one launch set
       if ((r = de::dense_dev(&c->cfg, dp.data() + bound[k], bound[k + 1] - bound[k],
                              dws + woff[k], woff[k + 1] - woff[k], sk,
-                             nch > 1 ? 1 : g_batch_streams, nch > 1, nch > 1)))
+                             nch > 1 ? 1 : g_batch_streams, nch > 1)))
         return r;
       DE_CUDA(cudaMemcpyAsync(&hstat[k], dws + woff[k], sizeof(int), cudaMemcpyDeviceToHost, sk));
       DE_CUDA(cudaEventRecord(c->ev_done[k], sk));

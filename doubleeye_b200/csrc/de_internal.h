@@ -78,11 +78,9 @@ struct Batch {
 
 // de_dense_dev with a bound on the parts a batch runs as on concurrent streams (1: one
 // launch set on `stream`); callers that already overlap batches of their own pass 1.
-// `reg_ring` keeps the column kernel's prefetch ring in registers (de_capi.cu);
 // `overlapped`: the caller runs other launch sets beside this one.
 int dense_dev(const de_cfg* cfg, const de_pair* pairs, int n, void* workspace,
-              size_t ws_bytes, cudaStream_t stream, int max_parts, bool reg_ring = false,
-              bool overlapped = false);
+              size_t ws_bytes, cudaStream_t stream, int max_parts, bool overlapped = false);
 
 // Device address of the no-allocation entry point's status word on the current device
 // (de_noalloc.cu); DE_OK or an error code already recorded for de_last_error().
