@@ -45,6 +45,7 @@
 // 124 -> 83, 640x480 D=256 179 -> 124, 1280x720 D=64 186 -> 137.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
@@ -153,7 +154,10 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ float fbits(uint32_t v) { return __uint_as_float(v); }
 
-template <int G>
+// RK: the filtered costs also go back to the volume, for the reverse match; the top-2
+// warps write them (from the chains, whose latency bounds the kernel, it cost 23 us more at
+// 848x480 D=64).
+template <int G, bool RK>
 __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, int cstride) {
   constexpr int DP = 64 * G;                          // Dpad
   constexpr int KW = DP / 2;                          // words per column
@@ -345,6 +349,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         wt.wait(&ofull[ob], (n / kOut) & 1);
         const uint32_t* row = outb + (ob * kBlk + r) * (2 * kRow);
         const uint4* seg = reinterpret_cast<const uint4*>(row + s * 32);
+        // RK: this lane's 32 costs of the row go back (where they came from: the chains are
+        // past them)
+        uint2* const vrow = RK && x < W - hw && y < yin && 32 * s < NCOL * DP
+                                ? reinterpret_cast<uint2*>(P.vol + (size_t(y) * W + x) * DP) + 8 * (s % (DP / 32))
+                                : nullptr;
         uint32_t p0 = 0, p1 = 0;
         // two more keys: the greatest of three, and their median against the second.
         // The keys are distinct, but for zeros (no candidate); a key names its own
@@ -361,6 +370,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
           const uint4 v = seg[i ^ s];
           add2(v.x, v.y);
           add2(v.z, v.w);
+          if (RK && vrow)
+            __stcg(vrow + (i ^ s), make_uint2(__byte_perm(v.x, v.y, 0x7632),
+                                              __byte_perm(v.z, v.w, 0x7632)));
         }
 #pragma unroll
         for (int o = 1; o < LPC; o <<= 1) {
@@ -440,7 +452,7 @@ size_t tm_smem(int G, int cstride) {
   return size_t(kStages + 2 * kOut) * kBlk * kRow * 4 + size_t(2) * ncol * cstride * 4;
 }
 
-template <int G>
+template <int G, bool RK>
 cudaError_t launch_g(const DevCfg& cfg, const Batch& b, int maxH, cudaStream_t s) {
   const int cstride = coef_stride(maxH, cfg.hh);
   const size_t sm = tm_smem(G, cstride);
@@ -448,9 +460,9 @@ cudaError_t launch_g(const DevCfg& cfg, const Batch& b, int maxH, cudaStream_t s
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const cudaError_t e = cudaFuncSetAttribute(
-      k_cols_tm<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+      k_cols_tm<G, RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
   if (e != cudaSuccess) return e;
-  k_cols_tm<G><<<std::min(b.cols_prefix[b.n], nsm), kThreads, sm, s>>>(cfg, b, cstride);
+  k_cols_tm<G, RK><<<std::min(b.cols_prefix[b.n], nsm), kThreads, sm, s>>>(cfg, b, cstride);
   return cudaGetLastError();
 }
 
@@ -460,7 +472,7 @@ bool cols_tm_fits(int H, int Dpad, int hh) {
   return tm_smem(Dpad / 64, coef_stride(H, hh)) <= size_t(224) << 10;
 }
 
-// `b0`: pairs of one disparity group that all fit (cols_tm_fits), without reverse keys.
+// `b0`: pairs of one disparity group that all fit (cols_tm_fits).
 cudaError_t launch_cols_tm(const DevCfg& cfg, const Batch& b0, cudaStream_t s) {
   thread_local Batch b;                               // tiles instead of columns
   b = b0;
@@ -473,12 +485,17 @@ cudaError_t launch_cols_tm(const DevCfg& cfg, const Batch& b0, cudaStream_t s) {
     maxH = std::max(maxH, b.p[i].H);
   }
   if (b.cols_prefix[b.n] == 0) return cudaSuccess;
-  switch (G) {
-    case 1: return launch_g<1>(cfg, b, maxH, s);
-    case 2: return launch_g<2>(cfg, b, maxH, s);
-    case 3: return launch_g<3>(cfg, b, maxH, s);
-    default: return launch_g<4>(cfg, b, maxH, s);
-  }
+  auto go = [&](auto rk) -> cudaError_t {
+    constexpr bool RK = decltype(rk)::value;
+    switch (G) {
+      case 1: return launch_g<1, RK>(cfg, b, maxH, s);
+      case 2: return launch_g<2, RK>(cfg, b, maxH, s);
+      case 3: return launch_g<3, RK>(cfg, b, maxH, s);
+      default: return launch_g<4, RK>(cfg, b, maxH, s);
+    }
+  };
+  // (a batch has reverse keys for all its pairs or for none)
+  return b.p[0].rkey ? go(std::true_type()) : go(std::false_type());
 }
 
 }  // namespace de

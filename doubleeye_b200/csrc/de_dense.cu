@@ -667,16 +667,10 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
         pk0 = hi;
         pk1 = max(pk1, sum - hi - lo);
       }
-      if (RK) {
-        const size_t rowo = size_t(y) * W + x - dmin - k0;
-#pragma unroll
-        for (int s = 0; s < KT; ++s)
-          if (s < nvalid)
-            atomicMax(P.rkey + rowo - s, (uint32_t(st[s]) << 8) | uint32_t(255 - k0 - s));
-      }
       uint32_t o[KW];
       pack_state(o);
       vstore<KW>(reinterpret_cast<uint32_t*>(rowbuf + k0), o);
+      if (RK && live) vstore<KW>(gcol + size_t(y) * grs, o);   // for the reverse match
     };
     auto merge_step = [&](uint32_t& pk0, uint32_t& pk1, int off) {
       const uint32_t o0 = __shfl_xor_sync(gmask, pk0, off, TPCP);
@@ -1670,16 +1664,46 @@ cudaError_t launch_cols_g(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
   }
 }
 
+// Reverse match (cfg.lrc): per right pixel the best key of all disparities that name it,
+// from the filtered costs that the column kernel wrote back.  A CTA takes kRkCols columns
+// of a row, whose candidates name at most kRkCols + D right pixels: shared-memory maxima,
+// then one global maximum each.  Bound by its one read of the volume.  One global atomic
+// per disparity, inside the column kernel's top-2, had that wait on them: 848x480 D=64
+// columns 157 us, now 81 and 35 here (59 with a thread per right pixel walking its
+// diagonal of the volume instead of the shared maxima).
+constexpr int kRkCols = 64;
+
+__global__ void __launch_bounds__(256) k_rkey(DevCfg cfg, DevPair P) {
+  __shared__ uint32_t best[kRkCols + 256];
+  const int W = P.W, D = P.D, KW = P.Dpad / 2, tid = threadIdx.x;
+  const int hw = cfg.hw, y = cfg.hh + blockIdx.y;
+  const int xb = hw + cfg.dmin + blockIdx.x * kRkCols, n = min(kRkCols, W - hw - xb);
+  for (int i = tid; i < kRkCols + 256; i += 256) best[i] = 0;
+  __syncthreads();
+  const uint32_t* v = reinterpret_cast<const uint32_t*>(P.vol) + (size_t(y) * W + xb) * KW;
+  for (int i = tid; i < n * KW; i += 256) {
+    const int c = i / KW, k = 2 * (i - c * KW), kmax = min(D - 1, xb + c - hw - cfg.dmin);
+    if (k > kmax) continue;
+    const uint32_t w = __ldcg(v + i);
+    const int at = c + 255 - k;                       // right pixel - (xb - dmin - 255)
+    atomicMax(&best[at], (w & 0xFFFFu) << 8 | uint32_t(255 - k));
+    if (k < kmax) atomicMax(&best[at - 1], (w >> 16) << 8 | uint32_t(254 - k));
+  }
+  __syncthreads();
+  uint32_t* out = P.rkey + size_t(y) * W;
+  for (int i = tid; i < kRkCols + 255; i += 256)
+    if (best[i]) atomicMax(out + (xb - cfg.dmin - 255 + i), best[i]);
+}
+
 // Whether a disparity group goes to the tensor-memory column kernel.  Its time is per
 // tile (512 bytes of an image row, one tile an SM at a time, about 27 us at 480 rows) and
 // it fills an SM; the streaming kernel's grows with the bytes once the GPU is full.  They
 // cross between 6 and 11 tiles an SM (one launch set, streaming / this, us): 1280x720
 // D=128 (4.3 tiles an SM) 241 / 226, two 848x480 D=128 pairs (5.7) 175 / 153, 1280x720
 // D=256 (8.6) 381 / 376, four 848x480 D=128 pairs (11.4) 287 / 289.  A launch set that
-// runs beside others needs the room this kernel takes from them, and the reverse-match
-// keys (lrc) make its top-2 warps wait on atomics (848x480 D=64: 169 / 214): both stream.
+// runs beside others needs the room this kernel takes from them: it streams.
 bool cols_tm_for(const DevCfg& cfg, const Batch& sub) {
-  if (!cfg.alone || sub.p[0].rkey) return false;
+  if (!cfg.alone) return false;
   const int per = std::max(1, 256 / sub.maxDpad);     // columns per tile
   int tiles = 0;
   for (int i = 0; i < sub.n; ++i) {
@@ -1713,6 +1737,12 @@ cudaError_t launch_cols(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
     const cudaError_t e = cols_tm_for(cfg, sub) ? launch_cols_tm(cfg, sub, s)
                                                 : launch_cols_g(cfg, sub, s);
     if (e != cudaSuccess) return e;
+    for (int i = 0; i < sub.n; ++i) {
+      const DevPair& P = sub.p[i];
+      const int ncols = P.W - 2 * cfg.hw - cfg.dmin, nrows = P.H - 2 * cfg.hh;
+      if (P.rkey && ncols > 0 && nrows > 0)
+        k_rkey<<<dim3((ncols + kRkCols - 1) / kRkCols, nrows), 256, 0, s>>>(cfg, P);
+    }
   }
   return cudaSuccess;
 }

@@ -105,7 +105,7 @@ cudaError_t launch_census(const DevCfg& cfg, const Batch& b, cudaStream_t s);
 cudaError_t launch_rows(const DevCfg& cfg, const Batch& b, cudaStream_t s);
 cudaError_t launch_cols(const DevCfg& cfg, const Batch& b, cudaStream_t s);
 // The column kernel with its forward results in tensor memory (de_cols.cu): one disparity
-// group's pairs, no reverse keys.  cols_tm_fits: its coefficient columns fit.
+// group's pairs.  cols_tm_fits: its coefficient columns fit.
 bool cols_tm_fits(int H, int Dpad, int hh);
 cudaError_t launch_cols_tm(const DevCfg& cfg, const Batch& b, cudaStream_t s);
 cudaError_t launch_solve(const DevCfg& cfg, const Batch& b, bool from_ref_layout,
