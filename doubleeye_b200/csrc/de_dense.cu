@@ -323,24 +323,25 @@ __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
     uint32_t* out = reinterpret_cast<uint32_t*>(P.vol + row * DP) + tid;
     int32_t f0 = kVolBias, f1 = kVolBias;
     {
-      uint64_t rprev = (xw - 1 - d0 >= 0) ? sR[xw - 1 - d0] : 0;    // chain k1's word
+      // Lanes may still be before their start: they score a clamped word and keep zero,
+      // without a branch, so that a step's loads and scores run ahead of the chain here
+      // too (with branches these 64 steps took 17 k clocks, the next 784 of an
+      // 848-pixel row 43 k).
+      uint64_t rprev = sR[max(xw - 1 - d0, 0)];       // chain k1's word
       int x = xw;
-      int xramp = min(xend, xw + 64);                 // lanes may still be before their start
+      int xramp = min(xend, xw + 64);
       xramp += (xramp - dmin) & 1;                    // the paired loop needs x - dmin even
       xramp = min(xramp, xend);
+#pragma unroll 8
       for (; x < xramp; ++x) {
         const int32_t a = sax[x];
-        const uint64_t lw = sLx[x];
-        int32_t v0 = kVolBias, v1 = kVolBias;
-        uint64_t rw = 0;
-        if (x - d0 >= hw) {
-          rw = sR[x - d0];
-          v0 = graded<PACKED, TS, 1>(lw, rw, tab, sLp, sRp, x, x - d0);
-        }
-        if (x - d0 - 1 >= hw) v1 = graded<PACKED, TS, 1>(lw, rprev, tab, sLp, sRp, x, x - d0 - 1);
+        const uint64_t lw = sLx[x], rw = sR[max(x - d0, 0)];
+        const int xr = max(x - d0, 0);
+        const int32_t v0 = graded<PACKED, TS, 1>(lw, rw, tab, sLp, sRp, x, xr);
+        const int32_t v1 = graded<PACKED, TS, 1>(lw, rprev, tab, sLp, sRp, x, max(xr - 1, 0));
         rprev = rw;
-        f0 = rf_step(v0, f0, a);
-        f1 = rf_step(v1, f1, a);
+        f0 = rf_step(x - d0 >= hw ? v0 : kVolBias, f0, a);
+        f1 = rf_step(x - d0 - 1 >= hw ? v1 : kVolBias, f1, a);
         out[x * XS] = pack2(f0, f1);
       }
       const uint64_t* rp = sR + (x - d0);

@@ -68,14 +68,17 @@ __device__ __forceinline__ int32_t graded(uint64_t lw, uint64_t rw, const void* 
   return static_cast<const uint16_t*>(tab)[ad * 64 + h];
 }
 
-// The table, by the whole CTA.
+// The table, by the whole CTA (any multiple of 32 threads).  A thread keeps its Hamming distance, so the parameter tables are read once per thread at
+// diverging addresses and then at one address for all (both per entry: 6-9 k clocks at
+// the start of every row CTA).
 template <int TS>
 __device__ __forceinline__ void fill_scores(const DevCfg& cfg, void* tab) {
   uint16_t* t16 = static_cast<uint16_t*>(tab);
-  for (int i = threadIdx.x; i < TS * 64; i += blockDim.x) {
-    const int m = i >> 6, h = i & 63;
-    t16[i] = uint16_t(kVolBias +
-                      ((int32_t(cfg.tbl[h]) * (1024 - cfg.wq) + int32_t(cfg.adt[m]) * cfg.wq) >> 10));
+  const int per = max(1, int(blockDim.x) >> 6);       // threads that share a distance
+  for (int h = threadIdx.x & 63; h < 64; h += blockDim.x) {
+    const int32_t c = int32_t(cfg.tbl[h]) * (1024 - cfg.wq);
+    for (int m = threadIdx.x >> 6; m < TS; m += per)
+      t16[m * 64 + h] = uint16_t(kVolBias + ((c + int32_t(cfg.adt[m]) * cfg.wq) >> 10));
   }
 }
 
