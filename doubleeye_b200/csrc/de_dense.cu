@@ -228,18 +228,18 @@ __global__ void __launch_bounds__(kCTX * kCTY) k_census_rows(DevCfg cfg, Batch b
 // the x-coefficients, read by both passes, are double-buffered.  Forward results go
 // to the volume with plain stores; the backward pass brings them back through a
 // ring of bulk copies, so no thread waits on a global load.
-// Backward ring: stages of kRowsChunk disparity-columns (x times Dpad, 4 KB), two or
+// Backward ring: stages of CB disparity-columns (x times Dpad; 2048 are 4 KB), two or
 // three in flight (NS).  The launcher takes two where that puts more rows in flight
 // at Dpad 64, else three, which hide the copies better.  Smaller stages lose more to
 // the per-stage barrier than an extra row gains (2 KB stages, nine rows per SM at
 // 848x480 D=128: rows 0.935 -> 0.971 ms per 16 pairs).
-constexpr int kRowsChunk = 2048;
+constexpr int kRowsChunk = 2048, kRowsChunkBig = 4096;
 
-template <bool PACKED, int TS, int G, int NS>
+template <bool PACKED, int TS, int G, int NS, int CB>
 __global__ void __launch_bounds__(32 * G, 8 / G) k_rows(DevCfg cfg, Batch b) {
   constexpr int DP = 64 * G;                          // Dpad
   constexpr int XS = DP / 2;                          // x stride in 32-bit words
-  constexpr int CH = kRowsChunk / DP;                 // x columns per backward chunk
+  constexpr int CH = CB / DP;                         // x columns per backward chunk
 
   constexpr size_t STAGE = size_t(CH) * DP * 2;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -1433,7 +1433,7 @@ __global__ void k_export(DevCfg cfg, Batch b) {
   }
 }
 
-size_t rows_smem(const Batch& b, int TS, int G, bool packed, int ring) {
+size_t rows_smem(const Batch& b, int TS, int G, bool packed, int ring, int chunk) {
   int cpm = 0, apm = 0, maxW = 0;
   for (int i = 0; i < b.n; ++i) {
     cpm = std::max(cpm, b.p[i].cpitch);
@@ -1443,7 +1443,7 @@ size_t rows_smem(const Batch& b, int TS, int G, bool packed, int ring) {
   size_t s = size_t(TS) * 64 * 2;
   s += size_t(cpm) * 16;
   s += 2 * ((size_t(apm) * 2 + 127) & ~size_t(127));
-  s += size_t(ring) * (kRowsChunk / (64 * G)) * (64 * G) * 2;
+  s += size_t(ring) * (chunk / (64 * G)) * (64 * G) * 2;
   if (!packed) s += size_t(maxW) * 2;
   return (s + 15) & ~size_t(15);
 }
@@ -1484,8 +1484,8 @@ int g_cols_async = 1;             // 8-row prefetch through shared memory (cp.as
 
 template <bool PACKED, int TS, int G>
 cudaError_t launch_rows_t(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
-  auto kern2 = k_rows<PACKED, TS, G, 2>;
-  auto kern3 = k_rows<PACKED, TS, G, 3>;
+  auto kern2 = k_rows<PACKED, TS, G, 2, kRowsChunk>;
+  auto kern3 = k_rows<PACKED, TS, G, 3, kRowsChunk>;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -1512,11 +1512,24 @@ cudaError_t launch_rows_t(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
     occ_cache.push_back({reinterpret_cast<const void*>(kern), sm, fit});
     return fit;
   };
-  const size_t sm2 = rows_smem(b, TS, G, PACKED, 2), sm3 = rows_smem(b, TS, G, PACKED, 3);
+  const size_t sm2 = rows_smem(b, TS, G, PACKED, 2, kRowsChunk);
+  const size_t sm3 = rows_smem(b, TS, G, PACKED, 3, kRowsChunk);
   const int per2 = std::max(1, std::min(fit_of(kern2, sm2), g_rows_ctas_per_sm));
   const int per3 = std::max(1, std::min(fit_of(kern3, sm3), g_rows_ctas_per_sm));
   const int items = b.rows_prefix[b.n];
   cudaError_t e;
+  // Few rows, all in flight whatever their footprint: 8 KB stages, half the barriers a row
+  // (one pair, rows: 848x480 D=128 74.1 -> 70.5 us, 640x480 D=256 98.9 -> 91.3; at Dpad 64,
+  // where a 4 KB stage is 32 columns already, no gain).
+  if constexpr (G >= 2) {
+    auto kernb = k_rows<PACKED, TS, G, 3, kRowsChunkBig>;
+    const size_t smb = rows_smem(b, TS, G, PACKED, 3, kRowsChunkBig);
+    if (items <= std::min(fit_of(kernb, smb), g_rows_ctas_per_sm) * nsm) {
+      if ((e = set_smem(kernb, smb)) != cudaSuccess) return e;
+      kernb<<<items, 32 * G, smb, s>>>(cfg, b);
+      return cudaGetLastError();
+    }
+  }
   if (G == 1 && std::min(items, per2 * nsm) > std::min(items, per3 * nsm)) {
     if ((e = set_smem(kern2, sm2)) != cudaSuccess) return e;
     kern2<<<std::min(items, per2 * nsm), 32 * G, sm2, s>>>(cfg, b);
