@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
   uint32_t* const outb = ring + kStages * kBlk * kRow;    // [kOut][kBlk][2 kRow] keys
   float* const coef = reinterpret_cast<float*>(outb + kOut * kBlk * 2 * kRow);  // [2][NCOL][cstride]
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages], ofull[kOut], oempty[kOut],
-      cfull[2], cempty[2];
+      cfull[2], cempty[2], cfirst;
   __shared__ uint32_t tmem;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int total = b.cols_prefix[b.n];
@@ -199,10 +199,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
     for (int i = 0; i < kStages; ++i) { mbar_init(&full[i], 32); mbar_init(&empty[i], 4); }
     for (int i = 0; i < kOut; ++i) { mbar_init(&ofull[i], 4); mbar_init(&oempty[i], 8); }
     for (int i = 0; i < 2; ++i) { mbar_init(&cfull[i], 1); mbar_init(&cempty[i], 4); }
+    mbar_init(&cfirst, 256);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) tm_alloc(&tmem, kTm);
-  if (warp >= 4 && warp < 12 && int(blockIdx.x) < total) load_coef(blockIdx.x, 0, tid - 128, 256);
   __syncthreads();
   Waiter wt{b.err};
 
@@ -228,7 +228,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
       const size_t rs = size_t(W) * KW;               // image row in words
       uint32_t* const gcol = reinterpret_cast<uint32_t*>(P.vol) + size_t(x) * KW + k0 / 2;
       const float* const cf = coef + ((it & 1) * NCOL + col) * cstride;
-      if (it > 0) wt.wait(&cfull[it & 1], ((it - (it & 1 ? 1 : 2)) >> 1) & 1);
+      if (it == 0) wt.wait(&cfirst, 0);
+      else wt.wait(&cfull[it & 1], ((it - (it & 1 ? 1 : 2)) >> 1) & 1);
       float f0 = 8388608.f + 32768.f, f1 = f0;
       auto step = [&](uint32_t c, float a) {
         const float c0 = fbits(__byte_perm(c, 0x4B000000u, 0x7610));
@@ -334,6 +335,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
   } else if (warp < 12) {
     // ---- the top-2 ------------------------------------------------------------------
     const int t = tid - 128;
+    if (int(blockIdx.x) < total) {                    // the first tile's coefficients
+      load_coef(blockIdx.x, 0, t, 256);
+      mbar_arrive(&cfirst);
+    }
     const int r = t >> 3, s = t & 7;                  // tile row, 32-disparity segment
     const int col = (G == 3) ? 0 : s / (2 * G);
     uint32_t n = 0;                                   // block count over the tiles
