@@ -514,7 +514,9 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int KT, int TPCP, int PF, int NT, bool AS = false>
+// RK: the filtered costs also go back to the volume, for the reverse match (a kernel of
+// its own: as a branch inside it cost the others 5% at 32 lanes a column).
+template <int KT, int TPCP, int PF, int NT, bool AS, bool RK>
 __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, Batch b) {
   static_assert((KT == 4 || KT % 8 == 0) && TPCP >= 1 && TPCP <= 32, "shape");
   static_assert(!AS || KT == 8, "the asynchronous ring moves 16 bytes a lane and row");
@@ -609,7 +611,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
     const int32_t a = aring[j];
     const int yn = y + PF;
     ring_fill(j, min(yn, ylast), dep);
-    aring[j] = ay[size_t(min(yn, H - 1)) * W];
+    aring[j] = ay[uint32_t(min(yn, H - 1)) * uint32_t(W)];
     step(c, a);
     if (live) {
       uint32_t o[KW];
@@ -620,7 +622,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
 #pragma unroll
   for (int j = 0; j < PF; ++j) {
     ring_fill(j, min(hh + j, ylast), 0u);
-    aring[j] = ay[size_t(min(hh + j, H - 1)) * W];
+    aring[j] = ay[uint32_t(min(hh + j, H - 1)) * uint32_t(W)];
   }
   int y0 = hh;
   for (; y0 + PF <= H; y0 += PF) {
@@ -637,15 +639,14 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
   for (; ys >= yin && ys >= hh; --ys) {
     uint32_t c[KW];
     fetch(ys, c);
-    step(c, ay[size_t(ys + 1) * W]);
+    step(c, ay[uint32_t(ys + 1) * uint32_t(W)]);
   }
   if (ys < hh) return;
   uint16_t* rowbufs[kRB];
 #pragma unroll
   for (int i = 0; i < kRB; ++i) rowbufs[i] = &sbuf[wib][i][gbase * KT];
   constexpr int kRowbufLast = TPCP * KT - 1;          // the group's last rowbuf entry
-  auto bwd_rows = [&](auto with_rkey) {
-    constexpr bool RK = decltype(with_rkey)::value;
+  {
     // One row: the filter step, the lane's top-2 keys, and its costs into a row
     // buffer (for the winner's neighbours).
     auto row_keys = [&](int y, int j, uint32_t& pk0, uint32_t& pk1, uint16_t* rowbuf) {
@@ -654,7 +655,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
       const int32_t a = aring[j];
       const int yn = y - PF;
       ring_fill(j, max(yn, 0), c[0]);
-      aring[j] = ay[size_t(max(yn + 1, 0)) * W];
+      aring[j] = ay[uint32_t(max(yn + 1, 0)) * uint32_t(W)];
       step(c, a);
       pk0 = 0;
       pk1 = 0;                                        // key 0 never displaces a candidate
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
       const int32_t vp = int32_t(rowbuf[min(kw + 1, kRowbufLast)]) - kVolBias;
       const int32_t nm = (kw >= 1) ? vm : -32768;
       const int32_t np = (kw >= 0 && kw + 1 <= kmax) ? vp : -32768;
-      const size_t i = size_t(y) * W + x;
+      const uint32_t i = uint32_t(y) * uint32_t(W) + uint32_t(x);   // (below 2^25)
       P.key0[i] = pk0;
       P.key1[i] = pk1;
       P.nb[i] = pk16(nm, np);
@@ -741,7 +742,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
 #pragma unroll
     for (int j = 0; j < PF; ++j) {
       ring_fill(j, max(ys - j, 0), 0u);
-      aring[j] = ay[size_t(max(ys - j + 1, 0)) * W];   // coefficient at y + 1
+      aring[j] = ay[uint32_t(max(ys - j + 1, 0)) * uint32_t(W)];   // coefficient at y + 1
     }
     int yb = ys;
     static_assert(PF % kRB == 0, "rows are taken kRB at a time");
@@ -752,9 +753,7 @@ __global__ void __launch_bounds__(NT, (AS ? 768 : 512) / NT) k_cols(DevCfg cfg, 
 #pragma unroll
     for (int j = 0; j < PF; ++j)
       if (yb - j >= hh) bwd(yb - j, j);
-  };
-  if (P.rkey) bwd_rows(std::integral_constant<bool, true>());
-  else bwd_rows(std::integral_constant<bool, false>());
+  }
   if constexpr (AS) cp_async_wait<0>();               // no copy outlives the CTA
 }
 
@@ -1520,11 +1519,12 @@ cudaError_t launch_rows_t(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
   cudaError_t e;
   // Few rows, all in flight whatever their footprint: 8 KB stages, half the barriers a row
   // (one pair, rows: 848x480 D=128 74.1 -> 70.5 us, 640x480 D=256 98.9 -> 91.3; at Dpad 64,
-  // where a 4 KB stage is 32 columns already, no gain).
+  // where a 4 KB stage is 32 columns already, no gain).  Not beside another launch set,
+  // which wants the shared memory (the uneven 12-pair batch 5.9 -> 6.06 ms with it).
   if constexpr (G >= 2) {
     auto kernb = k_rows<PACKED, TS, G, 3, kRowsChunkBig>;
     const size_t smb = rows_smem(b, TS, G, PACKED, 3, kRowsChunkBig);
-    if (items <= std::min(fit_of(kernb, smb), g_rows_ctas_per_sm) * nsm) {
+    if (cfg.alone && items <= std::min(fit_of(kernb, smb), g_rows_ctas_per_sm) * nsm) {
       if ((e = set_smem(kernb, smb)) != cudaSuccess) return e;
       kernb<<<items, 32 * G, smb, s>>>(cfg, b);
       return cudaGetLastError();
@@ -1581,8 +1581,8 @@ int get_solve_threads() { return g_solve_threads; }
 void set_rows_ctas_per_sm(int v) { g_rows_ctas_per_sm = v < 1 ? 1 : v; }
 int get_rows_ctas_per_sm() { return g_rows_ctas_per_sm; }
 
-template <int KT, int TPCP, int NT>
-cudaError_t launch_cols_nt(const DevCfg& cfg, const Batch& b0, const de_cfg_hw& hwc,
+template <int KT, int TPCP, int NT, bool RK>
+cudaError_t launch_cols_rk(const DevCfg& cfg, const Batch& b0, const de_cfg_hw& hwc,
                            cudaStream_t s) {
   constexpr int NCOL = NT / TPCP;
   thread_local Batch b;                               // tiles instead of columns
@@ -1599,27 +1599,35 @@ cudaError_t launch_cols_nt(const DevCfg& cfg, const Batch& b0, const de_cfg_hw& 
   const int pf = g_cols_pf ? g_cols_pf : (KT == 4 ? 16 : 8);
   if constexpr (KT == 4) {
     if (pf == 16) {
-      k_cols<KT, TPCP, 16, NT><<<tiles, NT, 0, s>>>(cfg, b);
+      k_cols<KT, TPCP, 16, NT, false, RK><<<tiles, NT, 0, s>>>(cfg, b);
       return cudaGetLastError();
     }
   }
   if constexpr (KT == 8) {
     if (pf >= 8 && cfg.cols_async) {                  // the ring in shared memory
       constexpr size_t ring_bytes = size_t(NT) * 8 * (KT / 2) * 4;
-      const cudaError_t e = set_smem(k_cols<KT, TPCP, 8, NT, true>, ring_bytes);
+      const cudaError_t e = set_smem(k_cols<KT, TPCP, 8, NT, true, RK>, ring_bytes);
       if (e != cudaSuccess) return e;
-      k_cols<KT, TPCP, 8, NT, true><<<tiles, NT, ring_bytes, s>>>(cfg, b);
+      k_cols<KT, TPCP, 8, NT, true, RK><<<tiles, NT, ring_bytes, s>>>(cfg, b);
       return cudaGetLastError();
     }
   }
   if constexpr (KT == 4 || (KT == 8 && TPCP <= 16)) {
     if (pf >= 8) {
-      k_cols<KT, TPCP, 8, NT><<<tiles, NT, 0, s>>>(cfg, b);
+      k_cols<KT, TPCP, 8, NT, false, RK><<<tiles, NT, 0, s>>>(cfg, b);
       return cudaGetLastError();
     }
   }
-  k_cols<KT, TPCP, 4, NT><<<tiles, NT, 0, s>>>(cfg, b);
+  k_cols<KT, TPCP, 4, NT, false, RK><<<tiles, NT, 0, s>>>(cfg, b);
   return cudaGetLastError();
+}
+
+// (a batch has reverse keys for all its pairs or for none)
+template <int KT, int TPCP, int NT>
+cudaError_t launch_cols_nt(const DevCfg& cfg, const Batch& b, const de_cfg_hw& hwc,
+                           cudaStream_t s) {
+  return b.p[0].rkey ? launch_cols_rk<KT, TPCP, NT, true>(cfg, b, hwc, s)
+                     : launch_cols_rk<KT, TPCP, NT, false>(cfg, b, hwc, s);
 }
 
 int g_cols_cta = 0;               // column-kernel CTA threads: 128, 256, or 0 = by shape
