@@ -40,7 +40,8 @@
 // multiply-add, which also zeroes a disparity with no candidate).
 //
 // What bounds it: the chains' latency, about 42 clocks a row down and 45 up with one
-// chain warp a scheduler.  Measured (column stage, one pair, streaming -> this):
+// chain warp a scheduler.  Measured (column stage, one pair, streaming -> this as first
+// written; the producers' start since took another 1-3 us off each):
 // 320x240 D=64 52 -> 24 us, 450x375 D=60 79 -> 30, 848x480 D=64 101 -> 56, 848x480 D=128
 // 124 -> 83, 640x480 D=256 179 -> 124, 1280x720 D=64 186 -> 137.
 #include <algorithm>
@@ -63,8 +64,9 @@ constexpr int kTm = 512;                 // tensor-memory columns: all of them
 constexpr int kThreads = 512;
 constexpr uint32_t kZero2 = 0x80008000u; // two zero scores
 
-// A poll that returns at once: the suspending form (try_wait) woke some waiters thousands
-// of clocks after their phase had completed.
+// A poll that returns at once.  Against the suspending form (try_wait) the column stage
+// took 23 instead of 27 us at 320x240 D=64, each launch timed by itself; no difference at
+// 848x480.
 __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
