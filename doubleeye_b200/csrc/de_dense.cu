@@ -1723,9 +1723,10 @@ __global__ void __launch_bounds__(256) k_rkey(DevCfg cfg, DevPair P) {
 // cross between 6 and 11 tiles an SM (one launch set, streaming / this, us): 1280x720
 // D=128 (4.3 tiles an SM) 241 / 226, two 848x480 D=128 pairs (5.7) 175 / 153, 1280x720
 // D=256 (8.6) 381 / 376, four 848x480 D=128 pairs (11.4) 287 / 289.  A launch set that
-// runs beside others needs the room this kernel takes from them: it streams.
+// runs beside others needs the room this kernel takes from them: it streams.  So does one
+// whose caller has set a column knob: those shape the streaming kernel.
 bool cols_tm_for(const DevCfg& cfg, const Batch& sub) {
-  if (!cfg.alone) return false;
+  if (!cfg.alone || g_cols_kt || g_cols_pf || g_cols_cta || !cfg.cols_async) return false;
   const int per = std::max(1, 256 / sub.maxDpad);     // columns per tile
   int tiles = 0;
   for (int i = 0; i < sub.n; ++i) {

@@ -165,9 +165,13 @@ DE_API int de_stage_times(float* ms, int n, int* launches);
  *   "rows_ctas_per_sm"  cap on row-kernel CTAs resident per SM (default 32, i.e.
  *                       as many as fit): fewer rows in flight keep each row's
  *                       forward pass in L2 for its backward pass
- *   "cols_kt"           disparities per lane in the column kernel: 4, 8, 16, or 0
- *                       to choose by batch size (default 0: 4 for batches too small
- *                       to fill the GPU with columns, else 8)
+ *   "cols_kt"           disparities per lane in the streaming column kernel: 4, 8, 16,
+ *                       or 0 to choose by batch size (default 0: 4 for batches too
+ *                       small to fill the GPU with columns, else 8).  With all four
+ *                       cols_* knobs at their defaults, a launch set that runs by
+ *                       itself and is small (about two 848x480 D=128 pairs) takes a
+ *                       column kernel of another form, which has no such shapes; any
+ *                       other setting of one of them means the streaming kernel
  *   "cols_pf"           image rows the column kernel's lanes load ahead of use:
  *                       4, 8, 16 (4 disparities per lane only), or 0 to choose by
  *                       shape (default 0: 16 at 4 disparities per lane, else 8; 16
