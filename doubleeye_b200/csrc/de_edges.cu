@@ -375,12 +375,13 @@ __global__ void __launch_bounds__(kSmallThreads) k_masda_small(SmallArgs s) {
     se[e] = a.se[e];
     beta[e] = rho[e] = 0.0;
   }
-  for (int k = tid; k < m; k += NT) { rptr[k] = 0; rbest[k] = 0; taken[k] = 0; s.assign[k] = -1; }
+  for (int k = tid; k < m; k += NT) { rptr[k] = 0; rbest[k] = 0; taken[k] = 0; }
   for (int k = tid; k < n; k += NT) { cptr[k] = 0; cbest[k] = 0; taken[m + k] = 0; }
-  if (__syncthreads_or(bad)) {                           // nothing is indexed by them
+  if (__syncthreads_or(bad)) {            // nothing is indexed by them, no output written
     if (tid == 0) *s.bad = 1;
     return;
   }
+  for (int k = tid; k < m; k += NT) s.assign[k] = -1;
   for (int e = tid; e < E; e += NT) {
     atomicAdd(&rptr[ei[e]], 1);
     atomicAdd(&cptr[ej[e]], 1);
