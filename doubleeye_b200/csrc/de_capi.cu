@@ -81,6 +81,30 @@ int set_error(int code, const char* fmt, ...) {
   return code;
 }
 
+// The limit is a property of the kernel on the device that all host threads share, so it is
+// always set to the most that the kernel can take: set to each launch's own size, a thread
+// with smaller work could lower it between another's set and launch, which then failed.
+cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  struct Most { const void* kernel; int dev; int bytes; };
+  thread_local std::vector<Most> known;               // (one entry a kernel and device)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int most = -1;
+  for (const Most& m : known)
+    if (m.kernel == kernel && m.dev == dev) most = m.bytes;
+  if (most < 0) {
+    cudaFuncAttributes fa;
+    if ((e = cudaFuncGetAttributes(&fa, kernel)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
+      return e;
+    most -= int(fa.sharedSizeBytes);
+    known.push_back({kernel, dev, most});
+  }
+  if (bytes > size_t(most)) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // Host-built tables, the same expressions as the reference so the values agree bit
 // for bit: the filter LUT core/tools/de_dense.cpp:533-546 (float, std::exp), the
 // score tables :1201-1223.

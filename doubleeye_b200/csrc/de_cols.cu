@@ -466,8 +466,7 @@ cudaError_t launch_g(const DevCfg& cfg, const Batch& b, int maxH, cudaStream_t s
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const cudaError_t e = cudaFuncSetAttribute(
-      k_cols_tm<G, RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+  const cudaError_t e = allow_smem(k_cols_tm<G, RK>, sm);
   if (e != cudaSuccess) return e;
   k_cols_tm<G, RK><<<std::min(b.cols_prefix[b.n], nsm), kThreads, sm, s>>>(cfg, b, cstride);
   return cudaGetLastError();

@@ -1450,11 +1450,6 @@ size_t rows_smem(const Batch& b, int TS, int G, bool packed, int ring, int chunk
 size_t solve_smem(int W) { return size_t(W) * 49 + 64; }
 size_t solve_px_smem(int W) { return size_t(W) * 44 + 8 + size_t(solve_big_max(W)) * 4 + 16; }
 
-template <typename K>
-cudaError_t set_smem(K kernel, size_t bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-}
-
 }  // namespace
 
 cudaError_t launch_census(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
@@ -1502,7 +1497,7 @@ cudaError_t launch_rows_t(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
     for (const Occ& o : occ_cache)
       if (o.k == reinterpret_cast<const void*>(kern) && o.sm == sm) return o.fit;
     int fit = 0;
-    if (set_smem(kern, sm) != cudaSuccess ||
+    if (allow_smem(kern, sm) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, 32 * G, sm) != cudaSuccess) {
       cudaGetLastError();
       fit = 1;
@@ -1525,16 +1520,16 @@ cudaError_t launch_rows_t(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
     auto kernb = k_rows<PACKED, TS, G, 3, kRowsChunkBig>;
     const size_t smb = rows_smem(b, TS, G, PACKED, 3, kRowsChunkBig);
     if (cfg.alone && items <= std::min(fit_of(kernb, smb), g_rows_ctas_per_sm) * nsm) {
-      if ((e = set_smem(kernb, smb)) != cudaSuccess) return e;
+      if ((e = allow_smem(kernb, smb)) != cudaSuccess) return e;
       kernb<<<items, 32 * G, smb, s>>>(cfg, b);
       return cudaGetLastError();
     }
   }
   if (G == 1 && std::min(items, per2 * nsm) > std::min(items, per3 * nsm)) {
-    if ((e = set_smem(kern2, sm2)) != cudaSuccess) return e;
+    if ((e = allow_smem(kern2, sm2)) != cudaSuccess) return e;
     kern2<<<std::min(items, per2 * nsm), 32 * G, sm2, s>>>(cfg, b);
   } else {
-    if ((e = set_smem(kern3, sm3)) != cudaSuccess) return e;
+    if ((e = allow_smem(kern3, sm3)) != cudaSuccess) return e;
     kern3<<<std::min(items, per3 * nsm), 32 * G, sm3, s>>>(cfg, b);
   }
   return cudaGetLastError();
@@ -1606,7 +1601,7 @@ cudaError_t launch_cols_rk(const DevCfg& cfg, const Batch& b0, const de_cfg_hw& 
   if constexpr (KT == 8) {
     if (pf >= 8 && cfg.cols_async) {                  // the ring in shared memory
       constexpr size_t ring_bytes = size_t(NT) * 8 * (KT / 2) * 4;
-      const cudaError_t e = set_smem(k_cols<KT, TPCP, 8, NT, true, RK>, ring_bytes);
+      const cudaError_t e = allow_smem(k_cols<KT, TPCP, 8, NT, true, RK>, ring_bytes);
       if (e != cudaSuccess) return e;
       k_cols<KT, TPCP, 8, NT, true, RK><<<tiles, NT, ring_bytes, s>>>(cfg, b);
       return cudaGetLastError();
@@ -1789,7 +1784,7 @@ cudaError_t launch_solve_w(const DevCfg& cfg, const Batch& b, bool from_ref, cud
     // 1024-thread CTA an SM (1500x1000 D=256 x4: 624 us with two, 591 with four)
     const int np = g_solve_threads ? (g_solve_threads == 512 ? 2 : 4) : (maxW <= 1024 ? 2 : 4);
     auto go = [&](auto kern, int np) -> cudaError_t {
-      const cudaError_t e2 = set_smem(kern, sm);
+      const cudaError_t e2 = allow_smem(kern, sm);
       if (e2 != cudaSuccess) return e2;
       kern<<<items, ((maxW + np - 1) / np + 31) / 32 * 32, sm, s>>>(cfg, b);
       return cudaGetLastError();
@@ -1801,7 +1796,7 @@ cudaError_t launch_solve_w(const DevCfg& cfg, const Batch& b, bool from_ref, cud
   }
   const size_t sm = solve_smem(maxW);
   auto go = [&](auto kern, int nt) -> cudaError_t {
-    cudaError_t e2 = set_smem(kern, sm);
+    cudaError_t e2 = allow_smem(kern, sm);
     if (e2 != cudaSuccess) return e2;
     kern<<<items, nt, sm, s>>>(cfg, b);
     return cudaSuccess;

@@ -788,7 +788,7 @@ int masda_edges_dev(const int64_t* ei, const int64_t* ej, const double* se, long
   a.E = E; a.m = m; a.n = n; a.lam = lam; a.gam = gam; a.damping = damping; a.eps = eps;
   if (small) {
     const size_t sm = small_smem(E, m, n);
-    cudaError_t e = cudaFuncSetAttribute(k_masda_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    cudaError_t e = allow_smem(k_masda_small, sm);
     if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, sizeof(int), s);
     if (e != cudaSuccess) return set_error(DE_ERR_CUDA, "small solve: %s", cudaGetErrorString(e));
     k_masda_small<<<1, kSmallThreads, sm, s>>>(SmallArgs{a, belief_out, assign, flag, iters});

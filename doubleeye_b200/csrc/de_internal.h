@@ -89,6 +89,14 @@ int noalloc_status_word(void** out);
 // Records a one-line reason for de_last_error() and returns code (de_capi.cu).
 int set_error(int code, const char* fmt, ...);
 
+// Lets `kernel` be launched with `bytes` of dynamic shared memory on the current device;
+// cudaErrorInvalidValue where that is more than it can take (de_capi.cu).
+cudaError_t allow_smem(const void* kernel, size_t bytes);
+template <typename K>
+cudaError_t allow_smem(K* kernel, size_t bytes) {
+  return allow_smem(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // Host-side preparation (de_capi.cu).
 void make_dev_cfg(const de_cfg& c, DevCfg* out);
 size_t pair_workspace_bytes(int W, int H, int D, bool lrc);

@@ -370,7 +370,7 @@ cudaError_t launch_prior(const DevCfg& cfg, const Batch& b, const float* prior, 
                                                            cfg.dmin + D - 1, band, mx, box);
   auto rows = [&](auto kern, size_t table) -> cudaError_t {
     const size_t sm = size_t(W) * 18 + table;
-    const cudaError_t e2 = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+    const cudaError_t e2 = allow_smem(kern, sm);
     if (e2 != cudaSuccess) return e2;
     kern<<<H, Dpad / 2, sm, s>>>(cfg, P, box);
     return cudaGetLastError();

@@ -1226,7 +1226,7 @@ int detect_fast_dev(const uint8_t* img, int W, int H, const de_det_cfg* c, de_ke
   else k_nms<<<sms * 8, 256, 0, s>>>(W, H, rad, d);
   const int capk = ((cell + 1) / 2) * ((cell + 1) / 2);
   const size_t sm = size_t(capk) * (sizeof(de_keypoint) + 2 * sizeof(int) + 5 * sizeof(float));
-  e = cudaFuncSetAttribute(k_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+  e = allow_smem(k_cells, sm);
   if (e != cudaSuccess) return set_error(DE_ERR_CUDA, "k_cells smem: %s", cudaGetErrorString(e));
   k_cells<<<cells, 256, sm, s>>>(img, W, H, cell, cols, keep, c->grad_window,
                                   c->min_local_std, c->subpixel, d);
@@ -1322,7 +1322,7 @@ int match_masda_dev(const de_keypoint* kl, const uint64_t* dl, int nl, const int
   const size_t avail = size_t(std::max(0, optin - int(fa.sharedSizeBytes))) & ~size_t(15);
   const size_t sm = std::max(std::max(size_t(N) * 8, size_t(1024)), avail);
   a.smem_bytes = int(sm);
-  e = cudaFuncSetAttribute(k_match, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+  e = allow_smem(k_match, sm);
   if (e != cudaSuccess) return set_error(DE_ERR_CUDA, "k_match smem: %s", cudaGetErrorString(e));
   k_match<<<1, 1024, sm, s>>>(a, m);
   e = cudaGetLastError();
