@@ -78,17 +78,24 @@ __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
-// Waits with a memory: after one has run out the rest return quickly.
+// The same for a whole warp: complete in every lane's eyes.  What follows from it is then
+// uniform, and the lanes stay together for the tensor-memory instructions, which want the
+// whole warp at the same one.
+__device__ __forceinline__ bool warp_poll(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_poll(bar, parity));
+}
+
+// Waits (of whole warps) with a memory: after one has run out the rest return quickly.
 struct Waiter {
   int* err;
   bool dead = false;
   __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) {
-    if (!mbar_poll(bar, parity)) dead = slow(bar, parity, err, dead);
+    if (!warp_poll(bar, parity)) dead = slow(bar, parity, err, dead);
   }
   static __device__ __noinline__ bool slow(uint64_t* bar, uint32_t parity, int* err, bool dead) {
     const int limit = dead ? 16 : kWaitLimit;
     for (int i = 0; i < limit; ++i)
-      if (mbar_poll(bar, parity)) return dead;
+      if (warp_poll(bar, parity)) return dead;
     if (err) atomicExch(err, 1);
     return true;
   }
@@ -97,14 +104,25 @@ struct Waiter {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
+// One arrival a warp, after all its lanes' accesses; predicated, so that no lane leaves the
+// others.
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  asm volatile(
+      "{\n .reg .pred p;\n setp.eq.s32 p, %1, 0;\n"
+      " @p mbarrier.arrive.shared::cta.b64 _, [%0];\n}" ::"r"(smem_addr(bar)), "r"(lane)
+      : "memory");
+}
 
 // Tensor memory as thread-private storage: lane i of a warp reads back the words it wrote.
 __device__ __forceinline__ void tm_alloc(uint32_t* slot, uint32_t cols) {     // one warp
+  __syncwarp();                          // (its first lane has set up the barriers)
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                    smem_addr(slot)), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tm_free(uint32_t base, uint32_t cols) {       // the same warp
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols)
                : "memory");
 }
@@ -251,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         if (blk + 1 < nbl) {
           take(nx);
           if (++st == kStages) { st = 0; sph ^= 1; }
-          ready = mbar_poll(&full[st], sph);
+          ready = warp_poll(&full[st], sph);
         }
         const int rows = yin - (hh + blk * kBlk);     // rows of the block with input
         if (rows < kBlk) {
@@ -274,18 +292,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
 #pragma unroll
           for (int r = 0; r < kBlk; ++r) __stcg(g + r * rs, c[r]);
         }
+        if (blk < nspill) __syncwarp();               // (lanes with and without a store)
         if (blk + 1 < nbl) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&empty[mine]);
+          warp_arrive(&empty[mine], lane);
         }
       };
       uint32_t ca[kBlk], cb[kBlk];
       if (nbl > 0) {
         take(ca);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[st]);
+        warp_arrive(&empty[st], lane);
         if (++st == kStages) { st = 0; sph ^= 1; }
-        ready = mbar_poll(&full[st], sph);
+        ready = warp_poll(&full[st], sph);
       }
       for (int blk = 0; blk < nb; blk += 2) {
         down(blk, ca, cb);
@@ -300,6 +317,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
           const uint32_t* g = gcol + size_t(hh + blk * kBlk) * rs;
 #pragma unroll
           for (int r = 0; r < kBlk; ++r) c[r] = (k0 <= kmax) ? __ldcg(g + r * rs) : kZero2;
+          __syncwarp();
         }
       };
       bool room = false;
@@ -311,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         uint32_t* o = outb + ob * (kBlk * 2 * kRow) + 2 * tid;
         const uint32_t mine = ob;
         if (++ob == kOut) { ob = 0; oph ^= 1; }
-        room = mbar_poll(&oempty[ob], oph ^ 1);
+        room = warp_poll(&oempty[ob], oph ^ 1);
 #pragma unroll
         for (int q = kBlk / 4 - 1; q >= 0; --q) {
           const float4 a = reinterpret_cast<const float4*>(cf + blk * kBlk)[q];
@@ -323,16 +341,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
           }
           next = a.x;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ofull[mine]);
+        warp_arrive(&ofull[mine], lane);
       };
       fetch(nb - 1, ca);
       for (int blk = nb - 1; blk >= 0; blk -= 2) {
         up(blk, ca, cb);
         if (blk > 0) up(blk - 1, cb, ca);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&cempty[it & 1]);
+      warp_arrive(&cempty[it & 1], lane);
     }
   } else if (warp < 12) {
     // ---- the top-2 ------------------------------------------------------------------
@@ -397,8 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         };
         const int32_t nm = p0 && kw >= 1 ? cost(kw - 1) : -32768;
         const int32_t np = p0 && kw + 1 < DP ? cost(kw + 1) : -32768;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&oempty[ob]);
+        warp_arrive(&oempty[ob], lane);
         if (s % LPC == 0 && x < W - hw && y < yin) {
           const size_t i = size_t(y) * W + x;
           P.key0[i] = __byte_perm(p0, 0u, 0x4320);    // v + 32768 << 8 | 255 - k
@@ -445,8 +460,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
       const int buf = it & 1;
       if (it >= 2) wt.wait(&cempty[buf], ((it - 2) >> 1) & 1);   // tile it - 2 is done
       load_coef(tile, buf, lane, 32);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&cfull[buf]);
+      warp_arrive(&cfull[buf], lane);
     }
   }
   __syncthreads();
