@@ -449,8 +449,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
                          smem_addr(&full[st])) : "memory");
       }
     }
-    // every copy has landed before the CTA ends: the last fill of each stage (an earlier
-    // one had landed before the chains freed its stage)
+    // every copy has landed before the CTA ends, also where a wait ran out above: each lane
+    // waits for its own, then for the arrivals of the last fill of each stage (an earlier one
+    // had landed before the chains freed its stage) with a limit of its own
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    wt.dead = false;
     for (uint32_t f = n > kStages ? n - kStages : 0; f < n; ++f)
       if (int(f % 3) == warp - 12) wt.wait(&full[f % kStages], (f / kStages) & 1);
   } else {
