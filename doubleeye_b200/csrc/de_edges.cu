@@ -291,13 +291,16 @@ __global__ void k_dec_flip(int* count, int cur) {
 }
 
 // ---- small problems: the whole solve in one CTA ---------------------------------------
-// A keypoint problem has a thousand or two edges; as grid-wide passes it is some 160
+// A keypoint problem has a thousand or two edges; as grid-wide passes it is some 180
 // launches of two or three microseconds and a host round trip per four decision rounds.
-// Here the edges, messages and both incidence lists sit in shared memory and a thread
-// takes a row or a column at a time: no launches, no atomics on messages.  The arithmetic
-// and the keys are the passes' own.  Bound by its block barriers (two a sweep) and
-// shared-memory latency.  1166 edges, 30 sweeps: masda() 1.33 ms as passes, 0.78 so (the
-// kernel 0.2).
+// Here the edges, messages and both incidence lists sit in shared memory and a row's or a
+// column's list is taken by a thread (up to kShort edges), eight lanes (up to kPiece) or
+// eight lanes a piece: no launches, no atomics on messages.  The arithmetic and the keys
+// are the passes' own.  Bound by its block barriers (two a sweep) and shared-memory
+// latency.  30 sweeps through de_masda_edges_dev, us (grid-wide passes / a thread a list of
+// any length / this): 300 edges 690 / 151 / 122, 1166 edges 673 / 273 / 224, 4096 edges on
+// 3000 + 3100 nodes 684 / 726 / 472; full 64 x 64 769 / 1156 / 334, 512 x 8 704 / 2699 / 482;
+// 4096 edges with skewed columns 706 / 6467 / 546.
 struct SmallArgs {
   BpArgs b;
   double* belief_out;
@@ -309,8 +312,17 @@ struct SmallArgs {
 constexpr int kSmallThreads = 512;
 constexpr long long kSmallEdges = 4096, kSmallNodes = 6144;
 
+// Who takes a list: a thread up to kShort edges, eight lanes up to kPiece, longer ones eight
+// lanes a piece.
+constexpr int kShort = 4, kPiece = 64, kMine = kPiece / 8;
+constexpr int kMaxMid = int(kSmallEdges / (kShort + 1));
+constexpr int kMaxPieces = int(kSmallEdges / kPiece + kSmallEdges / (kPiece + 1));
+struct Piece { uint16_t seg, lo, hi, first, n; };    // items [lo, hi); the list's pieces
+
 size_t small_smem(long long E, long long m, long long n) {
-  return size_t(E) * 32 + size_t(m + n + 2) * 4 + size_t(m + n) * 8 + 64;
+  return size_t(E) * 32 + size_t(m + n + 2) * 4 + size_t(m + n) * 8 + 64 +
+         size_t(kMaxPieces) * (2 * sizeof(u64) + sizeof(int) + 2 * sizeof(Piece)) +
+         size_t(kMaxMid) * 2 * sizeof(uint16_t);
 }
 bool small_fits(long long E, long long m, long long n) {
   return E > 0 && E <= kSmallEdges && m + n <= kSmallNodes && small_smem(E, m, n) <= size_t(220) << 10;
@@ -348,16 +360,37 @@ __device__ void cta_max_keys(u64& v0, u64& v1, u64 (*red)[32]) {
   __syncthreads();
 }
 
+// A list's greatest value, the greatest below it, and how many share the greatest.
+struct Top {
+  u64 m1 = kKeyNegInf, m2 = kKeyNegInf;
+  int cnt = 0;
+  __device__ __forceinline__ void join(u64 o1, u64 o2, int oc) {
+    cnt = o1 > m1 ? oc : (o1 == m1 ? cnt + oc : cnt);
+    m2 = max(max(m2, o2), o1 == m1 ? 0ull : min(o1, m1));
+    m1 = max(m1, o1);
+  }
+  __device__ __forceinline__ void put(u64 x) { join(x, 0ull, 1); }   // (0: no value)
+  __device__ __forceinline__ void join_group(unsigned mask) {        // of eight lanes
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+      join(__shfl_xor_sync(mask, m1, o), __shfl_xor_sync(mask, m2, o), __shfl_xor_sync(mask, cnt, o));
+  }
+};
+
 __global__ void __launch_bounds__(kSmallThreads) k_masda_small(SmallArgs s) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int sums[32];
   __shared__ u64 red[2][32];
+  __shared__ int s_n[4];                                 // lists of eight lanes, pieces
   const BpArgs& a = s.b;
   const int E = int(a.E), m = int(a.m), n = int(a.n), tid = threadIdx.x, NT = kSmallThreads;
   double* se = reinterpret_cast<double*>(smem);
   double* beta = se + E;
   double* rho = beta + E;
-  int* rptr = reinterpret_cast<int*>(rho + E);           // [m + 1]
+  u64* pm1 = reinterpret_cast<u64*>(rho + E);            // [kMaxPieces] the pieces' results
+  u64* pm2 = pm1 + kMaxPieces;
+  int* pcnt = reinterpret_cast<int*>(pm2 + kMaxPieces);
+  int* rptr = pcnt + kMaxPieces;                         // [m + 1]
   int* cptr = rptr + m + 1;                              // [n + 1]
   int* rbest = cptr + n + 1;                             // [m], fill counts first
   int* cbest = rbest + m;                                // [n]
@@ -366,6 +399,14 @@ __global__ void __launch_bounds__(kSmallThreads) k_masda_small(SmallArgs s) {
   uint16_t* ej = ei + E;
   uint16_t* rit = ej + E;
   uint16_t* cit = rit + E;
+  Piece* rpc = reinterpret_cast<Piece*>(cit + E);        // [kMaxPieces] of rows, of columns
+  Piece* cpc = rpc + kMaxPieces;
+  uint16_t* rmid = reinterpret_cast<uint16_t*>(cpc + kMaxPieces);   // [kMaxMid] lists
+  uint16_t* cmid = rmid + kMaxMid;
+  // groups of eight lanes, the last warps' first: the first warps have the short lists of a
+  // problem of a few hundred nodes
+  const int l8 = tid & 7, groups = NT >> 3, grp = groups - 1 - (tid >> 3);
+  const unsigned mask = 0xFFu << (tid & 24);
   int bad = 0;
   for (int e = tid; e < E; e += NT) {
     const int64_t i = a.ei[e], j = a.ej[e];
@@ -377,6 +418,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_masda_small(SmallArgs s) {
   }
   for (int k = tid; k < m; k += NT) { rptr[k] = 0; rbest[k] = 0; taken[k] = 0; }
   for (int k = tid; k < n; k += NT) { cptr[k] = 0; cbest[k] = 0; taken[m + k] = 0; }
+  if (tid < 4) s_n[tid] = 0;
   if (__syncthreads_or(bad)) {            // nothing is indexed by them, no output written
     if (tid == 0) *s.bad = 1;
     return;
@@ -393,37 +435,102 @@ __global__ void __launch_bounds__(kSmallThreads) k_masda_small(SmallArgs s) {
     rit[rptr[ei[e]] + atomicAdd(&rbest[ei[e]], 1)] = uint16_t(e);
     cit[cptr[ej[e]] + atomicAdd(&cbest[ej[e]], 1)] = uint16_t(e);
   }
+  auto cut = [&](const int* ptr, int nseg, uint16_t* mid, Piece* pc, int* count) {
+    for (int k = tid; k < nseg; k += NT) {
+      const int lo = ptr[k], hi = ptr[k + 1], len = hi - lo;
+      if (len > kShort && len <= kPiece) mid[atomicAdd(count, 1)] = uint16_t(k);
+      if (len <= kPiece) continue;
+      const int np = (len + kPiece - 1) / kPiece, first = atomicAdd(count + 1, np);
+      for (int i = 0; i < np; ++i)
+        pc[first + i] = Piece{uint16_t(k), uint16_t(lo + i * kPiece), uint16_t(min(hi, lo + (i + 1) * kPiece)),
+                              uint16_t(first), uint16_t(np)};
+    }
+  };
+  cut(rptr, m, rmid, rpc, s_n);
+  cut(cptr, n, cmid, cpc, s_n + 2);
   __syncthreads();
+  const int nrm = s_n[0], nrp = s_n[1], ncm = s_n[2], ncp = s_n[3];
   // one pass: out = (1 - d) * (s - max(floor, max_{segment, excl}(in))) + d * out
-  auto pass = [&](const int* ptr, const uint16_t* items, int nseg, const double* in, double* out,
-                  double floor) {
+  auto pass = [&](const int* ptr, const uint16_t* items, int nseg, const uint16_t* mid, int nmid,
+                  const Piece* pc, int np, const double* in, double* out, double floor) {
     u64 delta = okey(0.0);
+    // up to K items [lo, hi) of a list, `step` apart: their edges and keys (0: none), all
+    // loads before the first use; then their new messages
+    auto fetch = [&](int lo, int hi, int step, auto& e, auto& x, Top& t) {
+      constexpr int K = sizeof(x) / sizeof(u64);
+#pragma unroll
+      for (int i = 0; i < K; ++i) e[i] = lo + i * step < hi ? int(items[lo + i * step]) : -1;
+#pragma unroll
+      for (int i = 0; i < K; ++i) x[i] = e[i] >= 0 ? okey(in[e[i]]) : 0ull;
+#pragma unroll
+      for (int i = 0; i < K; ++i) t.put(x[i]);
+    };
+    auto update = [&](const auto& e, const auto& x, const Top& t) {
+      constexpr int K = sizeof(x) / sizeof(u64);
+      double sc[K], old[K];
+#pragma unroll
+      for (int i = 0; i < K; ++i) {
+        sc[i] = e[i] >= 0 ? se[e[i]] : 0.0;
+        old[i] = e[i] >= 0 ? out[e[i]] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < K; ++i) {
+        if (e[i] < 0) continue;
+        const double comp = fmax_np(floor, excluding(x[i], t.m1, t.m2, t.cnt));
+        const double v = (1.0 - a.damping) * (sc[i] - comp) + a.damping * old[i];
+        out[e[i]] = v;
+        delta = max(delta, okey(fabs(v - old[i])));
+      }
+    };
     for (int k = tid; k < nseg; k += NT) {
       const int lo = ptr[k], hi = ptr[k + 1];
-      u64 m1 = kKeyNegInf, m2 = kKeyNegInf;
-      int cnt = 0;
-      for (int q = lo; q < hi; ++q) {
-        const u64 x = okey(in[items[q]]);
-        if (x > m1) { m2 = m1; m1 = x; cnt = 1; }
-        else if (x == m1) ++cnt;
-        else m2 = max(m2, x);
+      if (hi - lo > kShort) continue;
+      int e[kShort];
+      u64 x[kShort];
+      Top t;
+      fetch(lo, hi, 1, e, x, t);
+      update(e, x, t);
+    }
+    int e[kMine];
+    u64 x[kMine];
+    for (int q = grp; q < nmid; q += groups) {
+      const int k = mid[q], lo = ptr[k], hi = ptr[k + 1];
+      Top t;
+      if (hi - lo <= 16) {
+        int e2[2];
+        u64 x2[2];
+        fetch(lo + l8, hi, 8, e2, x2, t);
+        t.join_group(mask);
+        update(e2, x2, t);
+      } else {
+        fetch(lo + l8, hi, 8, e, x, t);
+        t.join_group(mask);
+        update(e, x, t);
       }
-      for (int q = lo; q < hi; ++q) {
-        const int e = items[q];
-        const double comp = fmax_np(floor, excluding(okey(in[e]), m1, m2, cnt));
-        const double old = out[e];
-        const double v = (1.0 - a.damping) * (se[e] - comp) + a.damping * old;
-        out[e] = v;
-        delta = max(delta, okey(fabs(v - old)));
-      }
+    }
+    if (np == 0) return delta;
+    for (int p = grp; p < np; p += groups) {
+      Top t;
+      fetch(pc[p].lo + l8, pc[p].hi, 8, e, x, t);
+      t.join_group(mask);
+      if (l8 == 0) { pm1[p] = t.m1; pm2[p] = t.m2; pcnt[p] = t.cnt; }
+    }
+    __syncthreads();
+    for (int p = grp; p < np; p += groups) {
+      const Piece c = pc[p];
+      Top part, t;
+      fetch(c.lo + l8, c.hi, 8, e, x, part);
+      for (int q = c.first + l8; q < c.first + c.n; q += 8) t.join(pm1[q], pm2[q], pcnt[q]);
+      t.join_group(mask);
+      update(e, x, t);
     }
     return delta;
   };
   int it = 0;
   while (it < s.iters) {
-    u64 d0 = pass(rptr, rit, m, beta, rho, a.lam);
+    u64 d0 = pass(rptr, rit, m, rmid, nrm, rpc, nrp, beta, rho, a.lam);
     __syncthreads();
-    u64 d1 = pass(cptr, cit, n, rho, beta, a.gam);
+    u64 d1 = pass(cptr, cit, n, cmid, ncm, cpc, ncp, rho, beta, a.gam);
     cta_max_keys(d0, d1, red);                           // (barriers inside)
     const double d = fmax_np(dkey(d0), dkey(d1));
     if (tid == 0) a.hist[it] = d;
@@ -439,28 +546,60 @@ __global__ void __launch_bounds__(kSmallThreads) k_masda_small(SmallArgs s) {
     se[e] = (se[e] <= a.lam || !isfinite(b)) ? 0.0 : 1.0;
   }
   // greedy decision in rounds, as below
-  auto strongest = [&](const int* ptr, const uint16_t* items, int nseg, int own, int other,
+  auto strongest = [&](const int* ptr, const uint16_t* items, int nseg, const uint16_t* mid,
+                       int nmid, const Piece* pc, int np, int own, int other,
                        const uint16_t* to, int* out) {
     int any = 0;
-    for (int k = tid; k < nseg; k += NT) {
+    auto offer = [&](int e, int& best, u64& bk) {        // the first of the greatest
+      const u64 x = okey(rho[e]);
+      if (best < 0 || x > bk || (x == bk && e < best)) { best = e; bk = x; }
+    };
+    auto scan = [&](int lo, int hi, int step) {
       int best = -1;
       u64 bk = 0;
-      if (!taken[own + k])
-        for (int q = ptr[k]; q < ptr[k + 1]; ++q) {
-          const int e = items[q];
-          if (se[e] == 0.0 || taken[other + to[e]]) continue;
-          const u64 x = okey(rho[e]);
-          if (best < 0 || x > bk || (x == bk && e < best)) { best = e; bk = x; }
+      for (int q = lo; q < hi; q += step) {
+        const int e = items[q];
+        if (se[e] != 0.0 && !taken[other + to[e]]) offer(e, best, bk);
+      }
+      if (step == 8)
+        for (int o = 4; o > 0; o >>= 1) {
+          const int e = __shfl_xor_sync(mask, best, o);
+          if (e >= 0) offer(e, best, bk);
         }
+      return best;
+    };
+    auto put = [&](int k, int best) {
       out[k] = best;
       any |= best >= 0;
+    };
+    for (int k = tid; k < nseg; k += NT)
+      if (ptr[k + 1] - ptr[k] <= kShort) put(k, taken[own + k] ? -1 : scan(ptr[k], ptr[k + 1], 1));
+    for (int q = grp; q < nmid; q += groups) {
+      const int k = mid[q], best = taken[own + k] ? -1 : scan(ptr[k] + l8, ptr[k + 1], 8);
+      if (l8 == 0) put(k, best);
     }
+    if (np == 0) return any;
+    for (int p = grp; p < np; p += groups) {
+      const int best = taken[own + pc[p].seg] ? -1 : scan(pc[p].lo + l8, pc[p].hi, 8);
+      if (l8 == 0) pcnt[p] = best;
+    }
+    __syncthreads();
+    for (int p = tid; p < np; p += NT) {
+      const Piece c = pc[p];
+      if (p != c.first) continue;
+      int best = -1;
+      u64 bk = 0;
+      for (int q = p; q < p + c.n; ++q)
+        if (pcnt[q] >= 0) offer(pcnt[q], best, bk);
+      put(c.seg, best);
+    }
+    __syncthreads();                                     // (the pieces' results are used again)
     return any;
   };
   __syncthreads();
   for (int round = 0; round <= m; ++round) {
-    const int any = strongest(rptr, rit, m, 0, m, ej, rbest);
-    strongest(cptr, cit, n, m, 0, ei, cbest);
+    const int any = strongest(rptr, rit, m, rmid, nrm, rpc, nrp, 0, m, ej, rbest);
+    strongest(cptr, cit, n, cmid, ncm, cpc, ncp, m, 0, ei, cbest);
     if (!__syncthreads_or(any)) break;
     for (int k = tid; k < m; k += NT) {
       const int e = rbest[k];
