@@ -352,16 +352,20 @@ __global__ void __launch_bounds__(256) k_nms_w(int W, int H, int rad, DetWs d) {
 // Stage 3: one CTA per grid cell.  Texture floor, sub-pixel, strongest per_cell.  A cell of
 // 32 x 32 pixels keeps some 30 points, each of which needs a 49-pixel deviation and four
 // more responses: a thread per point and part, instead of all of a point's in one thread
-// (848x480: 57 -> 15.5 us).
-__global__ void __launch_bounds__(256) k_cells(const uint8_t* __restrict__ img, int W, int H,
+// (848x480: 57 -> 15.5 us).  kCellPart points at a time, so that a cell of 128 x 128 leaves
+// room for a second CTA on the SM: the ranking there is quadratic in the points (4096x2000
+// noise, suppression radius 1: the detection 6.15 ms with room for all parts, 3.98 so).
+constexpr int kCellPart = 256;
+
+__global__ void __launch_bounds__(kCellPart, 8) k_cells(const uint8_t* __restrict__ img, int W, int H,
                                                int cell, int cols, int keep, int gw,
                                                float min_std, int subpixel, DetWs d) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int cap = ((cell + 1) / 2) * ((cell + 1) / 2);
   de_keypoint* kp = reinterpret_cast<de_keypoint*>(smem);
+  // the pixels that suppression kept; from the front, those that pass the texture floor
   int* idx = reinterpret_cast<int*>(kp + cap);
-  int* found = idx + cap;                            // kept pixels before the texture floor
-  float* part = reinterpret_cast<float*>(found + cap);   // [cap][5] deviation, l, r, u, d
+  float* part = reinterpret_cast<float*>(idx + cap);   // [kCellPart][5] deviation, l, r, u, d
   __shared__ int s_n, s_found;
   const int c = blockIdx.x;
   const int x0 = (c % cols) * cell, y0 = (c / cols) * cell;
@@ -373,44 +377,47 @@ __global__ void __launch_bounds__(256) k_cells(const uint8_t* __restrict__ img, 
     const int i = (y0 + t / cw) * W + x0 + t % cw;
     if (d.state[i] != 2) continue;
     const int q = atomicAdd(&s_found, 1);
-    if (q < cap) found[q] = i;  // kept points are >= 2 apart, so q < cap always
+    if (q < cap) idx[q] = i;    // kept points are >= 2 apart, so q < cap always
   }
   __syncthreads();
   const int nf = min(s_found, cap), parts = subpixel ? 5 : 1;
-  for (int t = threadIdx.x; t < nf * parts; t += blockDim.x) {
-    const int q = t / parts, k = t % parts, xi = found[q] % W, yi = found[q] / W;
-    part[5 * q + k] = k == 0 ? local_std7(img, W, H, xi, yi)
-                             : shi_tomasi(img, W, H, xi + (k == 1 ? -1 : k == 2 ? 1 : 0),
-                                          yi + (k == 3 ? -1 : k == 4 ? 1 : 0), gw);
-  }
-  __syncthreads();
-  for (int f = threadIdx.x; f < nf; f += blockDim.x) {
-    const int i = found[f], xi = i % W, yi = i / W;
-    de_keypoint k;
-    k.x = float(xi);
-    k.y = float(yi);
-    k.response = d.resp[i];
-    k.local_std = part[5 * f];
-    if (k.local_std < min_std) continue;
-    if (subpixel) {
-      const float cc = k.response, l = part[5 * f + 1], r = part[5 * f + 2];
-      const float dxx = l - 2.f * cc + r;
-      if (fabsf(dxx) > 1e-12f) {
-        const float dd = 0.5f * (l - r) / dxx;
-        if (fabsf(dd) <= 0.5f) k.x += dd;
-      }
-      const float u = part[5 * f + 3], dn = part[5 * f + 4];
-      const float dyy = u - 2.f * cc + dn;
-      if (fabsf(dyy) > 1e-12f) {
-        const float dd = 0.5f * (u - dn) / dyy;
-        if (fabsf(dd) <= 0.5f) k.y += dd;
-      }
+  for (int f0 = 0; f0 < nf; f0 += kCellPart) {
+    const int nc = min(kCellPart, nf - f0);
+    for (int t = threadIdx.x; t < nc * parts; t += blockDim.x) {
+      const int q = t / parts, k = t % parts, xi = idx[f0 + q] % W, yi = idx[f0 + q] / W;
+      part[5 * q + k] = k == 0 ? local_std7(img, W, H, xi, yi)
+                               : shi_tomasi(img, W, H, xi + (k == 1 ? -1 : k == 2 ? 1 : 0),
+                                            yi + (k == 3 ? -1 : k == 4 ? 1 : 0), gw);
     }
-    const int q = atomicAdd(&s_n, 1);
-    kp[q] = k;
-    idx[q] = i;
+    const int f = threadIdx.x, i = f < nc ? idx[f0 + f] : 0;
+    __syncthreads();                                 // (the chunk's slots of idx are read)
+    if (f < nc && !(part[5 * f] < min_std)) {
+      const int xi = i % W, yi = i / W;
+      de_keypoint k;
+      k.x = float(xi);
+      k.y = float(yi);
+      k.response = d.resp[i];
+      k.local_std = part[5 * f];
+      if (subpixel) {
+        const float cc = k.response, l = part[5 * f + 1], r = part[5 * f + 2];
+        const float dxx = l - 2.f * cc + r;
+        if (fabsf(dxx) > 1e-12f) {
+          const float dd = 0.5f * (l - r) / dxx;
+          if (fabsf(dd) <= 0.5f) k.x += dd;
+        }
+        const float u = part[5 * f + 3], dn = part[5 * f + 4];
+        const float dyy = u - 2.f * cc + dn;
+        if (fabsf(dyy) > 1e-12f) {
+          const float dd = 0.5f * (u - dn) / dyy;
+          if (fabsf(dd) <= 0.5f) k.y += dd;
+        }
+      }
+      const int q = atomicAdd(&s_n, 1);
+      kp[q] = k;
+      idx[q] = i;
+    }
+    __syncthreads();
   }
-  __syncthreads();
   const int n = min(s_n, cap);
   for (int q = threadIdx.x; q < n; q += blockDim.x) {
     const float r = kp[q].response;
@@ -425,7 +432,7 @@ __global__ void __launch_bounds__(256) k_cells(const uint8_t* __restrict__ img, 
   if (threadIdx.x == 0) d.cellcnt[c] = min(n, keep);
 }
 
-// Exclusive scan of a[0..n) (global memory) by one CTA of NT threads; returns total.
+// Exclusive scan of a[0..n) (global or shared memory) by one CTA of NT threads; returns total.
 template <int NT>
 __device__ int cta_excl_scan(int* a, int n, int* warp_sums) {
   const int tid = threadIdx.x;
@@ -1225,10 +1232,11 @@ int detect_fast_dev(const uint8_t* img, int W, int H, const de_det_cfg* c, de_ke
   else if (rad <= 7) k_nms_w<7><<<sms * 8, 256, 0, s>>>(W, H, rad, d);
   else k_nms<<<sms * 8, 256, 0, s>>>(W, H, rad, d);
   const int capk = ((cell + 1) / 2) * ((cell + 1) / 2);
-  const size_t sm = size_t(capk) * (sizeof(de_keypoint) + 2 * sizeof(int) + 5 * sizeof(float));
+  const size_t sm = size_t(capk) * (sizeof(de_keypoint) + sizeof(int)) +
+                    size_t(std::min(capk, kCellPart)) * 5 * sizeof(float);
   e = allow_smem(k_cells, sm);
   if (e != cudaSuccess) return set_error(DE_ERR_CUDA, "k_cells smem: %s", cudaGetErrorString(e));
-  k_cells<<<cells, 256, sm, s>>>(img, W, H, cell, cols, keep, c->grad_window,
+  k_cells<<<cells, kCellPart, sm, s>>>(img, W, H, cell, cols, keep, c->grad_window,
                                   c->min_local_std, c->subpixel, d);
   k_det_emit<<<1, 1024, 0, s>>>(cells, keep, d, out, cap, n_out);
   e = cudaGetLastError();
