@@ -13,7 +13,7 @@
 //
 // Layout here: the plane-minor volume [y][x][Dpad] of the dense path.  Rows: a CTA per
 // image row with its census words in shared memory, a thread per pair of planes.
-// Columns: a group of lanes per column, four or eight planes a lane, whose top-2 are
+// Columns: a group of lanes per column, two, four or eight planes a lane, whose top-2 are
 // merged over the group.  Each plane's rectangle enters as its own filter coefficient: 0
 // at the rectangle's first pixel takes the input as it is, 2^15 outside carries the state
 // through, both exactly, so all planes of a thread step together without branches.
@@ -22,6 +22,7 @@
 // 2 (us, rows / columns): 888 / 1072 with a thread per plane, its loads in the chain, a
 // constant-memory score table and a compare-and-swap per insert; 200 / 247 now.
 #include <algorithm>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
@@ -117,7 +118,7 @@ __device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffff
 // The forward results go to the volume and come back eight words ahead.
 template <int TS>
 __global__ void __launch_bounds__(128) k_prior_rows(DevCfg cfg, DevPair P,
-                                                    const int* __restrict__ box) {
+                                                    const int* __restrict__ box, int apart) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int D = P.D, W = P.W, H = P.H, XS = P.Dpad / 2;
   const int y = blockIdx.x, tid = threadIdx.x;
@@ -153,58 +154,68 @@ __global__ void __launch_bounds__(128) k_prior_rows(DevCfg cfg, DevPair P,
   const int xj = warp_min(min(s0.n ? s0.last() : 1 << 28, s1.n ? s1.last() : 1 << 28));
   const int d0 = cfg.dmin + 2 * tid;
   uint32_t* out = reinterpret_cast<uint32_t*>(P.vol) + size_t(y) * W * XS + tid;
-  int32_t f0 = kVolBias, f1 = kVolBias;
-  // (a lane before its own rectangle reads a clamped right word that nothing looks at)
-  uint64_t rprev = sR[max(xs - 1 - d0, 0)];
+  // The lanes step over x together, so that a step's words are adjacent, or each from its own
+  // first position, where the planes' rectangles are short and far apart (a prior that
+  // slants across the image): `apart` times fewer steps at least.
+  const int own = warp_max(hi >= 0 ? hi - lo : 0);
+  auto passes = [&](auto by_lane) {
+    constexpr bool APART = decltype(by_lane)::value;
+    const int x0 = APART ? (hi >= 0 ? lo : xs) : xs, n = APART ? own : xe - xs;
+    auto at = [&](int x) { return APART ? min(x, W - 1) : x; };   // (past a lane's last)
+    int32_t f0 = kVolBias, f1 = kVolBias;
+    // (a lane before its own rectangle reads a clamped right word that nothing looks at)
+    uint64_t rprev = sR[max(x0 - 1 - d0, 0)];
 #pragma unroll 4
-  for (int x = xs; x <= xe; ++x) {
-    const uint64_t lw = sL[x], rw = sR[max(x - d0, 0)];
-    const int a = sax[x];
-    const int32_t c0 = graded<true, TS, 1>(lw, rw, tab, nullptr, nullptr, 0, 0);
-    const int32_t c1 = graded<true, TS, 1>(lw, rprev, tab, nullptr, nullptr, 0, 0);
-    rprev = rw;
-    int a0 = a, a1 = a;
-    if (x <= xi || x > xj) { a0 = s0.down(x, a); a1 = s1.down(x, a); }
-    f0 = rf_step(c0, f0, a0);
-    f1 = rf_step(c1, f1, a1);
-    if (x >= lo && x <= hi) out[size_t(x) * XS] = pack2(f0, f1);
-  }
-  // backward, eight words ahead
-  constexpr int PF = 8;
-  uint32_t cur[PF], nxt[PF];
-  auto fetch = [&](int x, uint32_t (&w)[PF]) {
-#pragma unroll
-    for (int i = 0; i < PF; ++i) w[i] = __ldcg(out + size_t(max(x - i, xs)) * XS);
-  };
-  fetch(xe - 1, cur);
-  for (int x = xe - 1; x >= xs; x -= PF) {
-    fetch(x - PF, nxt);
-#pragma unroll
-    for (int i = 0; i < PF; ++i) {
-      const int p = x - i;
-      if (p < xs) break;
-      const int a = sax[p + 1];
+    for (int t = 0; t <= n; ++t) {
+      const int x = x0 + t, xc = at(x);
+      const uint64_t lw = sL[xc], rw = sR[max(xc - d0, 0)];
+      const int a = sax[xc];
+      const int32_t c0 = graded<true, TS, 1>(lw, rw, tab, nullptr, nullptr, 0, 0);
+      const int32_t c1 = graded<true, TS, 1>(lw, rprev, tab, nullptr, nullptr, 0, 0);
+      rprev = rw;
       int a0 = a, a1 = a;
-      if (p < xi || p >= xj) { a0 = s0.up(p, a); a1 = s1.up(p, a); }
-      f0 = rf_step(int32_t(cur[i] & 0xFFFFu), f0, a0);
-      f1 = rf_step(int32_t(cur[i] >> 16), f1, a1);
-      if (p >= lo && p <= hi) out[size_t(p) * XS] = pack2(f0, f1);
+      if (APART || x <= xi || x > xj) { a0 = s0.down(x, a); a1 = s1.down(x, a); }
+      f0 = rf_step(c0, f0, a0);
+      f1 = rf_step(c1, f1, a1);
+      if (x >= lo && x <= hi) out[size_t(x) * XS] = pack2(f0, f1);
     }
+    // backward, eight words ahead
+    constexpr int PF = 8;
+    uint32_t cur[PF], nxt[PF];
+    auto fetch = [&](int t, uint32_t (&w)[PF]) {
 #pragma unroll
-    for (int i = 0; i < PF; ++i) cur[i] = nxt[i];
-  }
+      for (int i = 0; i < PF; ++i) w[i] = __ldcg(out + size_t(at(x0 + max(t - i, 0))) * XS);
+    };
+    fetch(n - 1, cur);
+    for (int t = n - 1; t >= 0; t -= PF) {
+      fetch(t - PF, nxt);
+#pragma unroll
+      for (int i = 0; i < PF; ++i) {
+        if (t < i) break;
+        const int p = x0 + t - i, a = sax[at(p + 1)];
+        int a0 = a, a1 = a;
+        if (APART || p < xi || p >= xj) { a0 = s0.up(p, a); a1 = s1.up(p, a); }
+        f0 = rf_step(int32_t(cur[i] & 0xFFFFu), f0, a0);
+        f1 = rf_step(int32_t(cur[i] >> 16), f1, a1);
+        if (p >= lo && p <= hi) out[size_t(p) * XS] = pack2(f0, f1);
+      }
+#pragma unroll
+      for (int i = 0; i < PF; ++i) cur[i] = nxt[i];
+    }
+  };
+  if (apart * own < xe - xs) passes(std::true_type());
+  else passes(std::false_type());
 }
 
-// Vertical passes and the masked top-2: TPC lanes a column, KT planes a lane: four planes
-// up to Dpad 128 (a warp per column: the most warps for one pair), else eight.
+// One column's vertical passes and masked top-2 by TPC lanes, each with planes k0 to k0 + KT.
 template <int KT, int TPC>
-__global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
-                                                    const int* __restrict__ box,
-                                                    const uint32_t* __restrict__ mx) {
-  constexpr int KW = KT / 2, PF = KT == 4 ? 8 : 4;     // words a lane and row, rows ahead
+__device__ __forceinline__ void prior_column(const DevCfg& cfg, const DevPair& P,
+                                             const int* __restrict__ box,
+                                             const uint32_t* __restrict__ mx, int x, int sub,
+                                             int k0) {
+  constexpr int KW = KT / 2, PF = KT <= 4 ? 8 : 4;     // words a lane and row, rows ahead
+  constexpr int MW = KT < 4 ? KT : 4;                  // interval words a load
   const int D = P.D, W = P.W, H = P.H, Dpad = P.Dpad;
-  const int sub = threadIdx.x % TPC, k0 = sub * KT;
-  const int x = cfg.hw + cfg.dmin + blockIdx.x * (128 / TPC) + threadIdx.x / TPC;
   Span sp[KT];
   uint32_t on = 0;                       // planes needed in this column
   int lo = 1 << 28, hi = -1, in_lo = -1, in_hi = 1 << 28;
@@ -234,7 +245,9 @@ __global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
   for (int i = 0; i < KT; ++i) f[i] = kVolBias;
   auto load = [&](int y, uint32_t (&w)[KW]) {
     const uint32_t* g = col + size_t(y) * st;
-    if constexpr (KW == 2) {
+    if constexpr (KW == 1) {
+      w[0] = __ldcg(g);
+    } else if constexpr (KW == 2) {
       const uint2 v = __ldcg(reinterpret_cast<const uint2*>(g));
       w[0] = v.x; w[1] = v.y;
     } else {
@@ -272,7 +285,9 @@ __global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
         f[i] = rf_step(int32_t(i & 1 ? c[i / 2] >> 16 : c[i / 2] & 0xFFFFu), f[i], co[i]);
       if (y >= lo && y <= hi) {
         uint32_t* g = col + size_t(y) * st;
-        if constexpr (KW == 2)
+        if constexpr (KW == 1)
+          *g = pack2(f[0], f[1]);
+        else if constexpr (KW == 2)
           *reinterpret_cast<uint2*>(g) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
         else
           *reinterpret_cast<uint4*>(g) = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]),
@@ -281,11 +296,19 @@ __global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
     }
   }
   // backward and the insert; a row's intervals come with its words
-  uint4 ring_m[PF][KT / 4];
-  auto load_m = [&](int y, uint4 (&m)[KT / 4]) {
+  uint32_t ring_m[PF][KT];
+  auto load_m = [&](int y, uint32_t (&m)[KT]) {
+    const uint32_t* g = mx + size_t(y) * Dpad + kc;
 #pragma unroll
-    for (int i = 0; i < KT / 4; ++i)
-      m[i] = reinterpret_cast<const uint4*>(mx + size_t(y) * Dpad + kc)[i];
+    for (int i = 0; i < KT; i += MW) {
+      if constexpr (MW == 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(g + i);
+        m[i] = v.x; m[i + 1] = v.y;
+      } else {
+        const uint4 v = *reinterpret_cast<const uint4*>(g + i);
+        m[i] = v.x; m[i + 1] = v.y; m[i + 2] = v.z; m[i + 3] = v.w;
+      }
+    }
   };
 #pragma unroll
   for (int j = 0; j < PF; ++j) {
@@ -299,11 +322,11 @@ __global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
     for (int j = 0; j < PF; ++j) {
       const int y = y0 - j;
       uint32_t c[KW];
-      uint4 m[KT / 4];
+      uint32_t m[KT];
 #pragma unroll
       for (int i = 0; i < KW; ++i) c[i] = ring[j][i];
 #pragma unroll
-      for (int i = 0; i < KT / 4; ++i) m[i] = ring_m[j][i];
+      for (int i = 0; i < KT; ++i) m[i] = ring_m[j][i];
       const int a = ring_a[j], yn = max(y - PF, ys);
       load(yn, ring[j]);
       load_m(yn, ring_m[j]);
@@ -320,8 +343,7 @@ __global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
 #pragma unroll
       for (int i = 0; i < KT; ++i) {
         f[i] = rf_step(int32_t(i & 1 ? c[i / 2] >> 16 : c[i / 2] & 0xFFFFu), f[i], co[i]);
-        const uint4 q = m[i / 4];
-        const uint32_t w = i % 4 == 0 ? q.x : i % 4 == 1 ? q.y : i % 4 == 2 ? q.z : q.w;
+        const uint32_t w = m[i];
         // (a needed plane's rows with an interval lie in its rectangle)
         const bool in = on >> i & 1 && x >= int(int16_t(w & 0xFFFFu)) &&
                         x <= (int32_t(w) >> 16);
@@ -347,6 +369,39 @@ __global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
   }
 }
 
+// Vertical passes and the masked top-2: TPC lanes a column, KT planes a lane: four planes
+// up to Dpad 128 (a warp per column: the most warps for one pair), else eight.  A warp whose
+// column's needed planes lie within 64 of each other (a slanted or smooth prior) takes two a
+// lane there (3000x200 D=256, slanted prior, band 0: the call 508 us without, 356 with).
+template <int KT, int TPC>
+__global__ void __launch_bounds__(128) k_prior_cols(DevCfg cfg, DevPair P,
+                                                    const int* __restrict__ box,
+                                                    const uint32_t* __restrict__ mx) {
+  const int sub = threadIdx.x % TPC, k0 = sub * KT;
+  const int x = cfg.hw + cfg.dmin + blockIdx.x * (128 / TPC) + threadIdx.x / TPC;
+  if constexpr (TPC == 32) {
+    int first = 1 << 28, last = -1;
+#pragma unroll
+    for (int i = 0; i < KT; ++i) {
+      const int k = k0 + i;
+      Rect r;
+      if (k >= P.D || !plane_rect(box, P.D, k, P.W, P.H, cfg.hw, cfg.hh, cfg.dmin + k, &r) ||
+          x < r.xlo || x >= r.xhi)
+        continue;
+      first = min(first, k);
+      last = k;
+    }
+    first = warp_min(first) & ~1;
+    last = warp_max(last);
+    if (last < 0) return;
+    if (last - first < 2 * TPC) {
+      prior_column<2, TPC>(cfg, P, box, mx, x, sub, first + 2 * sub);
+      return;
+    }
+  }
+  prior_column<KT, TPC>(cfg, P, box, mx, x, sub, k0);
+}
+
 }  // namespace
 
 size_t prior_ws_bytes(int W, int H, int D) {
@@ -368,11 +423,21 @@ cudaError_t launch_prior(const DevCfg& cfg, const Batch& b, const float* prior, 
   k_prior_init<<<1, 256, 0, s>>>(box, D, W, H);
   k_prior_mask<<<H, 256, size_t(2) * D * sizeof(int), s>>>(prior, W, H, D, Dpad, cfg.dmin,
                                                            cfg.dmin + D - 1, band, mx, box);
+  // Lanes that step apart write 32 sectors a step instead of four: no loss while the rows'
+  // chains are what bounds, so with few warps an SM, else only for so many fewer steps.
+  // Measured (one pair, slanted prior, us; together / apart): 60 warps at 3.5 times fewer
+  // steps 969 / 497; 400 at 4.1 times 338 / 264; 800 at 4.2 times 711 / 792, at 20 times
+  // 606 / 508; 2160 at 13 times 1707 / 1768, at 21 times 1682 / 1555; 4000 at 14 times
+  // 1222 / 1339.
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int apart = std::max(2, 2 * H * (Dpad / 64) / nsm);
   auto rows = [&](auto kern, size_t table) -> cudaError_t {
     const size_t sm = size_t(W) * 18 + table;
     const cudaError_t e2 = allow_smem(kern, sm);
     if (e2 != cudaSuccess) return e2;
-    kern<<<H, Dpad / 2, sm, s>>>(cfg, P, box);
+    kern<<<H, Dpad / 2, sm, s>>>(cfg, P, box, apart);
     return cudaGetLastError();
   };
   e = cfg.trunc < 16 ? rows(k_prior_rows<16>, ScoreTable<16, 1>::bytes())
