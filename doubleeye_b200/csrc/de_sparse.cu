@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
@@ -1062,57 +1063,63 @@ __global__ void __launch_bounds__(1024, 1) k_match(MatchArgs a, const MatchWs m)
       sd[p] = a.dr[j];
     }
   __syncthreads();
-  auto right_x = [&](int p) { return near ? sx[p] : a.kr[int(keys[p] & 0xffffffffu)].x; };
-  for (int i = tid; i < nl; i += NT) {
-    const de_keypoint l = a.kl[i];
-    const uint32_t klo = ord_f32(l.y - a.max_dy), khi = ord_f32(l.y + a.max_dy);
-    int lo = 0, hi = nr;
-    {
-      int p = 0, q = nr;
-      while (p < q) {
-        const int md = (p + q) >> 1;
-        if (uint32_t(keys[md] >> 32) < klo) p = md + 1; else q = md;
+  // (two forms of the loop: a choice at every access cost 6% where bands overflow)
+  auto candidates = [&](auto in_shared) {
+    constexpr bool NEAR = decltype(in_shared)::value;
+    auto right_x = [&](int p) { return NEAR ? sx[p] : a.kr[int(keys[p] & 0xffffffffu)].x; };
+    for (int i = tid; i < nl; i += NT) {
+      const de_keypoint l = a.kl[i];
+      const uint32_t klo = ord_f32(l.y - a.max_dy), khi = ord_f32(l.y + a.max_dy);
+      int lo = 0, hi = nr;
+      {
+        int p = 0, q = nr;
+        while (p < q) {
+          const int md = (p + q) >> 1;
+          if (uint32_t(keys[md] >> 32) < klo) p = md + 1; else q = md;
+        }
+        lo = p;
+        q = nr;
+        while (p < q) {
+          const int md = (p + q) >> 1;
+          if (!(khi < uint32_t(keys[md] >> 32))) p = md + 1; else q = md;
+        }
+        hi = p;
       }
-      lo = p;
-      q = nr;
-      while (p < q) {
-        const int md = (p + q) >> 1;
-        if (!(khi < uint32_t(keys[md] >> 32))) p = md + 1; else q = md;
-      }
-      hi = p;
-    }
-    const uint64_t dli = a.dl[i];
-    int* sj = m.slot_j + size_t(i) * maxc;
-    auto score = [&](int p, float x) {
-      de_keypoint r;
-      r.x = x;
-      r.y = unord_f32(uint32_t(keys[p] >> 32));
-      return pair_score(l, r, dli, near ? sd[p] : a.dr[int(keys[p] & 0xffffffffu)], a, i);
-    };
-    int ns = 0;
-    for (int p = lo; p < hi; ++p) {
-      const float x = right_x(p), d = l.x - x;
-      if (d < a.min_disp || d > a.max_disp) continue;
-      if (ns < maxc) sj[ns] = int(keys[p] & 0xffffffffu);
-      ++ns;
-    }
-    if (ns > maxc) {          // best maxc by score, in score order (ties: band order)
+      const uint64_t dli = a.dl[i];
+      int* sj = m.slot_j + size_t(i) * maxc;
+      auto score = [&](int p, float x) {
+        de_keypoint r;
+        r.x = x;
+        r.y = unord_f32(uint32_t(keys[p] >> 32));
+        return pair_score(l, r, dli, NEAR ? sd[p] : a.dr[int(keys[p] & 0xffffffffu)], a, i);
+      };
+      int ns = 0;
       for (int p = lo; p < hi; ++p) {
         const float x = right_x(p), d = l.x - x;
         if (d < a.min_disp || d > a.max_disp) continue;
-        const float s = score(p, x);
-        int rank = 0;
-        for (int q = lo; q < hi && rank < maxc; ++q) {
-          const float xq = right_x(q), dq = l.x - xq;
-          if (dq < a.min_disp || dq > a.max_disp) continue;
-          const float sq = score(q, xq);
-          rank += (sq > s || (sq == s && q < p)) ? 1 : 0;
-        }
-        if (rank < maxc) sj[rank] = int(keys[p] & 0xffffffffu);
+        if (ns < maxc) sj[ns] = int(keys[p] & 0xffffffffu);
+        ++ns;
       }
+      if (ns > maxc) {          // best maxc by score, in score order (ties: band order)
+        for (int p = lo; p < hi; ++p) {
+          const float x = right_x(p), d = l.x - x;
+          if (d < a.min_disp || d > a.max_disp) continue;
+          const float s = score(p, x);
+          int rank = 0;
+          for (int q = lo; q < hi && rank < maxc; ++q) {
+            const float xq = right_x(q), dq = l.x - xq;
+            if (dq < a.min_disp || dq > a.max_disp) continue;
+            const float sq = score(q, xq);
+            rank += (sq > s || (sq == s && q < p)) ? 1 : 0;
+          }
+          if (rank < maxc) sj[rank] = int(keys[p] & 0xffffffffu);
+        }
+      }
+      m.cnt[i] = min(ns, maxc);
     }
-    m.cnt[i] = min(ns, maxc);
-  }
+  };
+  if (near) candidates(std::true_type());
+  else candidates(std::false_type());
   __syncthreads();
   const int E = cta_excl_scan<1024>(m.cnt, nl, warp_sums);
   int N2 = 1;
