@@ -78,24 +78,23 @@ __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
-// The same for a whole warp: complete in every lane's eyes.  What follows from it is then
-// uniform, and the lanes stay together for the tensor-memory instructions, which want the
-// whole warp at the same one.
-__device__ __forceinline__ bool warp_poll(uint64_t* bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_poll(bar, parity));
-}
-
-// Waits (of whole warps) with a memory: after one has run out the rest return quickly.
+// Waits with a memory: after one has run out the rest return quickly.
 struct Waiter {
   int* err;
   bool dead = false;
   __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) {
-    if (!warp_poll(bar, parity)) dead = slow(bar, parity, err, dead);
+    if (!mbar_poll(bar, parity)) dead = slow(bar, parity, err, dead);
+  }
+  // By a whole warp, whose lanes leave together: the tensor-memory instructions want them at
+  // the same one.  `seen`: what this lane's poll ahead of the wait returned.
+  __device__ __forceinline__ void wait_warp(uint64_t* bar, uint32_t parity, bool seen = false) {
+    if (__all_sync(0xffffffffu, seen) || __all_sync(0xffffffffu, mbar_poll(bar, parity))) return;
+    dead = __any_sync(0xffffffffu, slow(bar, parity, err, dead));
   }
   static __device__ __noinline__ bool slow(uint64_t* bar, uint32_t parity, int* err, bool dead) {
     const int limit = dead ? 16 : kWaitLimit;
     for (int i = 0; i < limit; ++i)
-      if (warp_poll(bar, parity)) return dead;
+      if (mbar_poll(bar, parity)) return dead;
     if (err) atomicExch(err, 1);
     return true;
   }
@@ -248,8 +247,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
       const size_t rs = size_t(W) * KW;               // image row in words
       uint32_t* const gcol = reinterpret_cast<uint32_t*>(P.vol) + size_t(x) * KW + k0 / 2;
       const float* const cf = coef + ((it & 1) * NCOL + col) * cstride;
-      if (it == 0) wt.wait(&cfirst, 0);
-      else wt.wait(&cfull[it & 1], ((it - (it & 1 ? 1 : 2)) >> 1) & 1);
+      if (it == 0) wt.wait_warp(&cfirst, 0);
+      else wt.wait_warp(&cfull[it & 1], ((it - (it & 1 ? 1 : 2)) >> 1) & 1);
       float f0 = 8388608.f + 32768.f, f1 = f0;
       auto step = [&](uint32_t c, float a) {
         const float c0 = fbits(__byte_perm(c, 0x4B000000u, 0x7610));
@@ -257,9 +256,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         f0 = __fadd_rd(__fmaf_rd(a, f0 - c0, c0 + kHalf), kUp);
         f1 = __fadd_rd(__fmaf_rd(a, f1 - c1, c1 + kHalf), kUp);
       };
-      bool ready = false;                             // the next stage has landed
+      bool ready = false;                             // the next stage has landed (polled ahead)
       auto take = [&](uint32_t (&c)[kBlk]) {          // the next block's words
-        if (!ready) wt.wait(&full[st], sph);
+        wt.wait_warp(&full[st], sph, ready);
         const uint32_t* s = ring + st * (kBlk * kRow) + tid;
 #pragma unroll
         for (int r = 0; r < kBlk; ++r) c[r] = s[r * kRow];
@@ -269,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         if (blk + 1 < nbl) {
           take(nx);
           if (++st == kStages) { st = 0; sph ^= 1; }
-          ready = warp_poll(&full[st], sph);
+          ready = mbar_poll(&full[st], sph);
         }
         const int rows = yin - (hh + blk * kBlk);     // rows of the block with input
         if (rows < kBlk) {
@@ -302,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         take(ca);
         warp_arrive(&empty[st], lane);
         if (++st == kStages) { st = 0; sph ^= 1; }
-        ready = warp_poll(&full[st], sph);
+        ready = mbar_poll(&full[st], sph);
       }
       for (int blk = 0; blk < nb; blk += 2) {
         down(blk, ca, cb);
@@ -325,11 +324,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
         float next = cf[blk * kBlk + kBlk];           // coefficient at y + 1
         if (blk >= nspill) tm_wait_ld(c);
         if (blk > 0) fetch(blk - 1, nx);
-        if (!room) wt.wait(&oempty[ob], oph ^ 1);
+        wt.wait_warp(&oempty[ob], oph ^ 1, room);
         uint32_t* o = outb + ob * (kBlk * 2 * kRow) + 2 * tid;
         const uint32_t mine = ob;
         if (++ob == kOut) { ob = 0; oph ^= 1; }
-        room = warp_poll(&oempty[ob], oph ^ 1);
+        room = mbar_poll(&oempty[ob], oph ^ 1);
 #pragma unroll
         for (int q = kBlk / 4 - 1; q >= 0; --q) {
           const float4 a = reinterpret_cast<const float4*>(cf + blk * kBlk)[q];
