@@ -1688,13 +1688,23 @@ cudaError_t launch_cols_g(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
 // per disparity, inside the column kernel's top-2, had that wait on them: 848x480 D=64
 // columns 157 us, now 81 and 35 here (59 with a thread per right pixel walking its
 // diagonal of the volume instead of the shared maxima).
-constexpr int kRkCols = 64;
+//
+// A pair of kRkOwn CTAs or more has a launch of its own; kRkShare smaller ones or more share
+// one, where a CTA looks its pair up (64 pairs of 160x120 in one call 821 us with a launch
+// each, 622 so; for large pairs the look-up costs 4-6% of the call, for one or two small ones
+// 2-4 us).
+constexpr int kRkCols = 64, kRkOwn = 2048, kRkShare = 4;
 
-__global__ void __launch_bounds__(256) k_rkey(DevCfg cfg, DevPair P) {
+__host__ __device__ inline int rkey_tiles(const DevCfg& cfg, int W) {      // CTAs a row
+  const int cols = W - 2 * cfg.hw - cfg.dmin;
+  return cols > 0 ? (cols + kRkCols - 1) / kRkCols : 0;
+}
+
+__device__ __forceinline__ void rkey_tile(const DevCfg& cfg, const DevPair& P, int tile, int row) {
   __shared__ uint32_t best[kRkCols + 256];
   const int W = P.W, D = P.D, KW = P.Dpad / 2, tid = threadIdx.x;
-  const int hw = cfg.hw, y = cfg.hh + blockIdx.y;
-  const int xb = hw + cfg.dmin + blockIdx.x * kRkCols, n = min(kRkCols, W - hw - xb);
+  const int hw = cfg.hw, y = cfg.hh + row;
+  const int xb = hw + cfg.dmin + tile * kRkCols, n = min(kRkCols, W - hw - xb);
   for (int i = tid; i < kRkCols + 256; i += 256) best[i] = 0;
   __syncthreads();
   const uint32_t* v = reinterpret_cast<const uint32_t*>(P.vol) + (size_t(y) * W + xb) * KW;
@@ -1710,6 +1720,41 @@ __global__ void __launch_bounds__(256) k_rkey(DevCfg cfg, DevPair P) {
   uint32_t* out = P.rkey + size_t(y) * W;
   for (int i = tid; i < kRkCols + 255; i += 256)
     if (best[i]) atomicMax(out + (xb - cfg.dmin - 255 + i), best[i]);
+}
+
+__global__ void __launch_bounds__(256) k_rkey(DevCfg cfg, DevPair P) {
+  rkey_tile(cfg, P, blockIdx.x, blockIdx.y);
+}
+
+__global__ void __launch_bounds__(256) k_rkey_pairs(DevCfg cfg, Batch b) {   // cols_prefix: CTAs
+  const int pi = find_pair(b.cols_prefix, b.n, blockIdx.x);
+  const int item = blockIdx.x - b.cols_prefix[pi], tiles = rkey_tiles(cfg, b.p[pi].W);
+  rkey_tile(cfg, b.p[pi], item % tiles, item / tiles);
+}
+
+cudaError_t launch_rkey(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
+  thread_local Batch few;
+  few.n = 0;
+  few.cols_prefix[0] = 0;
+  for (int i = 0; i < b.n; ++i) {
+    const DevPair& P = b.p[i];
+    const int tiles = rkey_tiles(cfg, P.W), rows = std::max(0, P.H - 2 * cfg.hh);
+    if (tiles * rows >= kRkOwn) {
+      k_rkey<<<dim3(tiles, rows), 256, 0, s>>>(cfg, P);
+    } else {
+      few.p[few.n++] = P;
+      few.cols_prefix[few.n] = few.cols_prefix[few.n - 1] + tiles * rows;
+    }
+  }
+  const int n = few.cols_prefix[few.n];
+  if (few.n >= kRkShare && n > 0) {
+    k_rkey_pairs<<<n, 256, 0, s>>>(cfg, few);
+  } else {
+    for (int i = 0; i < few.n; ++i)
+      if (few.cols_prefix[i + 1] > few.cols_prefix[i])
+        k_rkey<<<dim3(rkey_tiles(cfg, few.p[i].W), few.p[i].H - 2 * cfg.hh), 256, 0, s>>>(cfg, few.p[i]);
+  }
+  return cudaGetLastError();
 }
 
 // Whether a disparity group goes to the tensor-memory column kernel.  Its time is per
@@ -1755,12 +1800,8 @@ cudaError_t launch_cols(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
     const cudaError_t e = cols_tm_for(cfg, sub) ? launch_cols_tm(cfg, sub, s)
                                                 : launch_cols_g(cfg, sub, s);
     if (e != cudaSuccess) return e;
-    for (int i = 0; i < sub.n; ++i) {
-      const DevPair& P = sub.p[i];
-      const int ncols = P.W - 2 * cfg.hw - cfg.dmin, nrows = P.H - 2 * cfg.hh;
-      if (P.rkey && ncols > 0 && nrows > 0)
-        k_rkey<<<dim3((ncols + kRkCols - 1) / kRkCols, nrows), 256, 0, s>>>(cfg, P);
-    }
+    if (!sub.p[0].rkey) continue;
+    if (const cudaError_t e2 = launch_rkey(cfg, sub, s); e2 != cudaSuccess) return e2;
   }
   return cudaSuccess;
 }

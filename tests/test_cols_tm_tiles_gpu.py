@@ -50,3 +50,23 @@ def test_unequal_heights(D, lrc):
         _lib.set_param("batch_streams", saved)
     for g, (L, R) in zip(got, pairs):
         check({k: v.cpu().numpy() for k, v in g.items()}, kw, L, R)
+
+
+def test_reverse_match_of_uneven_pairs():
+    """One launch set whose pairs differ in size and group: seven small ones in one group
+    (two of them without candidates), and one in another."""
+    from doubleeye_b200 import _lib, dense
+    kw = dict(dmin=30, dmax=90, iters=1, lrc=1)
+    sizes = [(36, 20, 0), (200, 9, 0), (37, 50, 0), (330, 41, 0), (30, 8, 0), (101, 77, 0),
+             (230, 30, 220), (64, 64, 0)]
+    pairs = [images(W, H, 60, W + H) for W, H, _ in sizes]
+    saved = _lib.get_param("batch_streams")
+    try:
+        _lib.set_param("batch_streams", 1)
+        got = dense.DenseMatcher(dense.Cfg(**kw)).match_batch(
+            [(*(torch.from_numpy(i).cuda() for i in p), d) for p, (_, _, d) in zip(pairs, sizes)],
+            cand=True)
+    finally:
+        _lib.set_param("batch_streams", saved)
+    for g, (L, R), (_, _, d) in zip(got, pairs, sizes):
+        check({k: v.cpu().numpy() for k, v in g.items()}, dict(kw, dmax=d or 90), L, R)
