@@ -795,11 +795,11 @@ __device__ __forceinline__ float fit_offset(const DevCfg& cfg, float c0, int32_t
 
 // One pixel's outputs: disparity, reverse-match residuals (dense_solve.hpp:442-451,
 // core/tools/de_dense.cpp:1581-1597), candidate planes, confidence.  rev(xr): the
-// disparity index of the best candidate that names right pixel xr, -1 if none.
-template <typename Rev>
+// disparity index of the best candidate that names right pixel xr, -1 if none; kd(j): that of
+// the pixel's own candidate j.
+template <typename Disp, typename Rev>
 __device__ __forceinline__ void put_pixel(const DevCfg& cfg, const DevPair& P, size_t row, int x,
-                                          int n, float s1, float s2, int k0, int k1, float dl,
-                                          Rev rev) {
+                                          int n, float s1, float s2, float dl, Disp kd, Rev rev) {
   const int W = P.W, dmin = cfg.dmin;
   const size_t WH = size_t(W) * P.H;
   if (P.disp) P.disp[row + x] = dl;
@@ -820,8 +820,8 @@ __device__ __forceinline__ void put_pixel(const DevCfg& cfg, const DevPair& P, s
   if (P.cand) {
     P.cand[row + x] = s1;
     P.cand[WH + row + x] = s2;
-    P.cand[2 * WH + row + x] = n > 0 ? float(dmin + k0) : kNegBig;
-    P.cand[3 * WH + row + x] = n > 1 ? float(dmin + k1) : kNegBig;
+    P.cand[2 * WH + row + x] = n > 0 ? float(dmin + kd(0)) : kNegBig;
+    P.cand[3 * WH + row + x] = n > 1 ? float(dmin + kd(1)) : kNegBig;
     P.cand[4 * WH + row + x] = lrc;
     P.cand[5 * WH + row + x] = lrc2;
   }
@@ -1119,7 +1119,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1536 / kSolveThreads) k_solve(D
       }
       dl = float(dmin + s_cd[2 * x + j]) + off;
     }
-    put_pixel(cfg, P, row, x, n, cs2.x, cs2.y, s_cd[2 * x], s_cd[2 * x + 1], dl,
+    put_pixel(cfg, P, row, x, n, cs2.x, cs2.y, dl, [&](int j) { return int(s_cd[2 * x + j]); },
               [&](int xr) { return int(s_rev[xr]); });
   };
   // the neighbour words of a thread's pixels, four at a time, loads first
@@ -1399,8 +1399,8 @@ __global__ void __launch_bounds__(MAXT, MAXT > 512 ? 1 : NP == 2 ? 3 : 2) k_solv
       const float off = cfg.subpixel && bj[i] == 0 ? fit_offset(cfg, cs[i][0], lo16(nb[i]), hi16(nb[i])) : 0.f;
       dl = float(dmin + (bj[i] ? k1 : k0)) + off;
     }
-    put_pixel(cfg, P, row, x, int(key[i][0] != 0) + int(key[i][1] != 0), cs[i][0], cs[i][1], k0, k1,
-              dl, [&](int xr) {
+    put_pixel(cfg, P, row, x, int(key[i][0] != 0) + int(key[i][1] != 0), cs[i][0], cs[i][1],
+              dl, [&](int j) { return j ? k1 : k0; }, [&](int xr) {
                 const uint32_t r = s_rev[xr];
                 return r ? (8191 - int(r & 8191u)) / 2 - dmin - xr : -1;
               });
