@@ -4,13 +4,16 @@ The kernels leave the arithmetic fixed; these knobs only change how work is laid
 onto the GPU, so every setting gives bit-identical results:
 
   rows_ctas_per_sm  resident row-kernel CTAs per SM (persistent grid size)
-  cols_kt           column-kernel tile shape: disparities per lane (0 = by batch size)
-  cols_pf           column-kernel prefetch depth: image rows loaded ahead of use
-  cols_cta          column-kernel threads per CTA (0 = by batch size)
-  solve_threads     threads per row in the row solve, the BP schedule's width (0 = by
-                    row width)
+  cols_kt           streaming column kernel: disparities per lane (0 = by batch size)
+  cols_pf           streaming column kernel: image rows loaded ahead of use
+  cols_cta          streaming column kernel: threads per CTA (0 = by batch size)
+  solve_threads     row solve: two pixels a thread (512), four (256), 0 = by row width
   batch_streams     parts a batch runs as on concurrent streams
-  cols_async        column-kernel prefetch through shared memory (1) or registers (0)
+  cols_async        streaming column kernel: prefetch through shared memory (1) or
+                    registers (0)
+
+A single pair of usual size takes a column kernel of another form while the four cols_*
+knobs are at their defaults; any other setting of one of them means the streaming kernel.
 
 ``tune`` times a batch under a coordinate-descent search over these values (CUDA
 events, warm-up first) and returns the fastest setting; ``Tuner`` caches the choice
@@ -30,7 +33,7 @@ KNOBS = {
     "cols_kt": [0, 4, 8, 16],
     "cols_pf": [0, 4, 8, 16],
     "cols_cta": [0, 128, 256],
-    "solve_threads": [0, 128, 256, 512],
+    "solve_threads": [0, 256, 512],          # (128 is the same launch as 256)
     "batch_streams": [1, 2, 3, 4],
     "cols_async": [1, 0],
 }

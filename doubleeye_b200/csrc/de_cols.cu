@@ -27,7 +27,7 @@
 //   4-11  the top-2: eight lanes a row, 32 disparities each, so no shuffle chain is in
 //         the filter's way.
 // Block hand-offs are mbarriers; every wait is bounded (a wait that runs out sets the
-// batch status word, later ones give up at once, copies in flight are drained and the
+// batch status word, later ones give up at once, each lane waits for its own copies and the
 // tensor memory is freed).
 //
 // The step runs on the FP32 pipe, exactly.  With u = v + 32768 (the volume's bias) and
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cols_tm(DevCfg cfg, Batch b, in
       }
     }
   } else if (warp < 15) {
-    // ---- producers: three warps take the stages in turn -------------------------------------------------------------------
+    // ---- producers: three warps take the stages in turn -----------------------------
     uint32_t n = 0;                                   // blocks so far, over the tiles
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
       const int pi = find_pair(b.cols_prefix, b.n, tile);

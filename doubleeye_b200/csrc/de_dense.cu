@@ -867,9 +867,8 @@ __device__ __forceinline__ void block_excl_scan(int* a, int n, int* warp_sums) {
   __syncthreads();
 }
 
-// At most 40 registers (six 256-thread CTAs' worth, no spills): the solve still fits
-// five rows per SM by shared memory, and the registers it leaves free let the other
-// launch set's kernels run beside it (the 16-pair batch 2.381 -> 2.376 ms).
+// At most 40 registers (six 256-thread CTAs' worth, no spills); shared memory allows five
+// rows of 848 pixels per SM.
 template <bool REF_LAYOUT, int kSolveThreads>
 __global__ void __launch_bounds__(kSolveThreads, 1536 / kSolveThreads) k_solve(DevCfg cfg, Batch b) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -1472,7 +1471,7 @@ cudaError_t launch_census(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
 
 struct de_cfg_hw { int hw, dmin; };
 int g_rows_ctas_per_sm = 32;      // upper bound on row CTAs per SM (rows in flight)
-int g_solve_threads = 0;          // threads per row in the solve: 128, 256, 512, 0 = by width
+int g_solve_threads = 0;          // 512: two pixels a thread in the solve, 128 or 256: four, 0 = by width
 int g_cols_pf = 0;                // rows the column kernel prefetches: 4, 8, 16, 0 = by shape
 int g_cols_async = 1;             // 8-row prefetch through shared memory (cp.async)
 
@@ -1761,10 +1760,14 @@ cudaError_t launch_rkey(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
 // tile (512 bytes of an image row, one tile an SM at a time, about 27 us at 480 rows) and
 // it fills an SM; the streaming kernel's grows with the bytes once the GPU is full.  They
 // cross between 6 and 11 tiles an SM (one launch set, streaming / this, us): 1280x720
-// D=128 (4.3 tiles an SM) 241 / 226, two 848x480 D=128 pairs (5.7) 175 / 153, 1280x720
-// D=256 (8.6) 381 / 376, four 848x480 D=128 pairs (11.4) 287 / 289.  A launch set that
-// runs beside others needs the room this kernel takes from them: it streams.  So does one
-// whose caller has set a column knob: those shape the streaming kernel.
+// D=128 (4.3 tiles an SM) 241 / 226, two 848x480 D=128 pairs (5.7, with the knob
+// batch_streams at 1: by default a call of several pairs is two sets) 175 / 153, 1280x720
+// D=256 (8.6) 381 / 376, four 848x480 D=128 pairs (11.4) 287 / 289.  Launch sets of one call
+// that run beside each other need the room this kernel takes from them (16 pairs 2150 us
+// streaming, 2418 with it): they stream.  Separate callers need not: one, two and four
+// threads that each match single 848x480 D=128 pairs take 228 / 196, 171 / 157 and 156 / 150
+// us a pair.  A caller that has set a column knob gets the streaming kernel, which those
+// shape.
 bool cols_tm_for(const DevCfg& cfg, const Batch& sub) {
   if (!cfg.alone || g_cols_kt || g_cols_pf || g_cols_cta || !cfg.cols_async) return false;
   const int per = std::max(1, 256 / sub.maxDpad);     // columns per tile
@@ -1807,8 +1810,7 @@ cudaError_t launch_cols(const DevCfg& cfg, const Batch& b, cudaStream_t s) {
 }
 
 // `b` holds pairs of one width class.  Shared memory is sized for the class's widest
-// row; threads per row come from the knob, or by width (512 above 1024 pixels, else
-// 256).
+// row.
 cudaError_t launch_solve_w(const DevCfg& cfg, const Batch& b, bool from_ref, cudaStream_t s) {
   const int items = b.solve_prefix[b.n];
   if (items == 0) return cudaSuccess;

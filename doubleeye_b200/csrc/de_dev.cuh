@@ -68,9 +68,9 @@ __device__ __forceinline__ int32_t graded(uint64_t lw, uint64_t rw, const void* 
   return static_cast<const uint16_t*>(tab)[ad * 64 + h];
 }
 
-// The table, by the whole CTA (any multiple of 32 threads).  A thread keeps its Hamming distance, so the parameter tables are read once per thread at
-// diverging addresses and then at one address for all (both per entry: 6-9 k clocks at
-// the start of every row CTA).
+// The table, by the whole CTA (any multiple of 32 threads).  A thread keeps its Hamming
+// distance, so the parameter tables are read once per thread at diverging addresses and
+// then at one address for all (both per entry: 6-9 k clocks at the start of every row CTA).
 template <int TS>
 __device__ __forceinline__ void fill_scores(const DevCfg& cfg, void* tab) {
   uint16_t* t16 = static_cast<uint16_t*>(tab);

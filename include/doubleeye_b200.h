@@ -179,14 +179,16 @@ DE_API int de_stage_times(float* ms, int n, int* launches);
  *   "cols_cta"          column-kernel threads per CTA: 128, 256, or 0 to choose by
  *                       batch size (default 0: 128 for batches of a few 848x480
  *                       pairs or less, else 256)
- *   "solve_threads"     threads per image row in the row solve: 128, 256, 512, or
- *                       0 to choose by row width (default 0: 512 for rows wider
- *                       than 1024 pixels, else 256)
+ *   "solve_threads"     how the row solve spreads a row: 512 gives a thread two
+ *                       pixels (four above 2048 pixels), 128 and 256 four, 0 chooses
+ *                       by row width (default 0: two up to 1024 pixels, else four).
+ *                       For caller-made candidates (de_solve_dev), and for a lambda
+ *                       or gamma beyond +-1e6 or a damping outside 0..1, it is the
+ *                       threads per image row (0: 512 above 1024 pixels, else 256)
  *   "cols_async"        1 (default) or 0: at 8 disparities per lane the column
  *                       kernel's 8-row prefetch goes through shared memory by
  *                       asynchronous copies (fewer registers, so more warps and more
- *                       room for a concurrent launch set) instead of a register ring;
- *                       the host context's chunked batches keep the register ring
+ *                       room for a concurrent launch set) instead of a register ring
  *   "batch_streams"     1..4 (default 2): de_dense_dev runs a batch of several
  *                       pairs as that many parts, pairs taken in turn, each part's
  *                       launch set on its own stream forked from and joined back to
