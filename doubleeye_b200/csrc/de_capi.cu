@@ -85,8 +85,11 @@ int set_error(int code, const char* fmt, ...) {
 // always set to the most that the kernel can take: set to each launch's own size, a thread
 // with smaller work could lower it between another's set and launch, which then failed.
 cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  // what a kernel can take on a device, looked up once a thread (the oldest entry gives way)
   struct Most { const void* kernel; int dev; int bytes; };
-  thread_local std::vector<Most> known;               // (one entry a kernel and device)
+  constexpr int kKnown = 64;
+  thread_local Most known[kKnown] = {};
+  thread_local int looked_up = 0;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -99,7 +102,7 @@ cudaError_t allow_smem(const void* kernel, size_t bytes) {
     if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
       return e;
     most -= int(fa.sharedSizeBytes);
-    known.push_back({kernel, dev, most});
+    known[looked_up++ % kKnown] = Most{kernel, dev, most};
   }
   if (bytes > size_t(most)) return cudaErrorInvalidValue;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
